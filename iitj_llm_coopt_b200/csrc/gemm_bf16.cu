@@ -269,44 +269,53 @@ EncodeTiledFn encode_fn() {
 }
 
 struct MapKey {
-    const void* ptr; uint64_t rows, cols; uint32_t box_rows, box_cols;
+    const void* ptr; uint64_t rows, cols; uint32_t box_rows, box_cols, element;
     bool operator==(const MapKey& o) const {
-        return ptr == o.ptr && rows == o.rows && cols == o.cols && box_rows == o.box_rows && box_cols == o.box_cols;
+        return ptr == o.ptr && rows == o.rows && cols == o.cols && box_rows == o.box_rows && box_cols == o.box_cols && element == o.element;
     }
 };
 struct MapKeyHash {
     size_t operator()(const MapKey& k) const {
         return std::hash<const void*>()(k.ptr) ^ ((size_t)k.rows * 1000003u) ^ ((size_t)k.cols * 7919u) ^
-               ((size_t)k.box_rows << 20) ^ ((size_t)k.box_cols << 40);
+               ((size_t)k.box_rows << 20) ^ ((size_t)k.box_cols << 40) ^ ((size_t)k.element << 50);
     }
 };
 std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;
 std::mutex g_maps_mutex;
 
-}  // namespace
-
-int llm_tensor_map_2d(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols, CUtensorMap* out) {
+// `element`: bytes of an element, 2 (bfloat16) or 4 (float32).
+int tensor_map(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols, uint32_t element, CUtensorMap* out) {
     std::lock_guard<std::mutex> lock(g_maps_mutex);
-    const MapKey key{ptr, rows, cols, box_rows, box_cols};
+    const MapKey key{ptr, rows, cols, box_rows, box_cols, element};
     auto it = g_maps.find(key);
     if (it != g_maps.end()) { *out = it->second; return 0; }
     EncodeTiledFn fn = encode_fn();
     if (!fn) LLM_FAIL(-2, "tensor map: cuTensorMapEncodeTiled is not available from this driver");
-    if (((uintptr_t)ptr & 15) || (cols % 8)) LLM_FAIL(-1, "tensor map: matrices must be 16-byte aligned with a row length that is a multiple of 8 (got %llu)", (unsigned long long)cols);
-    if (box_cols * 2 > 128 || box_rows > 256) LLM_FAIL(-1, "tensor map: box %u x %u does not fit the 128-byte swizzle", box_cols, box_rows);
+    if (((uintptr_t)ptr & 15) || (cols * element % 16)) LLM_FAIL(-1, "tensor map: matrices must be 16-byte aligned with a row length that is a multiple of %u (got %llu)", 16 / element, (unsigned long long)cols);
+    if (box_cols * element > 128 || box_rows > 256) LLM_FAIL(-1, "tensor map: box %u x %u does not fit the 128-byte swizzle", box_cols, box_rows);
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    cuuint64_t strides[1] = {(cuuint64_t)cols * element};
     cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     cuuint32_t elem[2] = {1, 1};
     CUtensorMap m;
-    CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, elem,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CUresult r = fn(&m, element == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr),
+                    dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) LLM_FAIL(-2, "tensor map: cuTensorMapEncodeTiled failed with code %d", (int)r);
     if (g_maps.size() > 4096) g_maps.clear();
     g_maps.emplace(key, m);
     *out = m;
     return 0;
+}
+
+}  // namespace
+
+int llm_tensor_map_2d(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols, CUtensorMap* out) {
+    return tensor_map(ptr, rows, cols, box_rows, box_cols, 2, out);
+}
+
+int llm_tensor_map_2d_f32(const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols, CUtensorMap* out) {
+    return tensor_map(ptr, rows, cols, box_rows, box_cols, 4, out);
 }
 
 namespace {

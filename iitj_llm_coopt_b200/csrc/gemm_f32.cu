@@ -1,6 +1,7 @@
-// float32 matrix products on the CUDA cores: y = x . W^T with x [M, K] and W [N, K], both
-// row-major (the layout of F.linear in engine/model.py:194, 208, 210-211, 218).  This is the
-// true 32-bit path: plain FMA, no tensor cores, no TF32.  Each output element is the sum
+// float32 matrix products on the CUDA cores, for rows that do not start on 16-byte boundaries (all others:
+// gemm_f32_tc.cu): y = x . W^T with x [M, K] and W [N, K], both
+// row-major (the layout of F.linear in engine/model.py:194, 208, 210-211, 218).
+// Plain FMA, no tensor cores.  Each output element is the sum
 // over k = 0 .. K-1 in that order, so a row's result does not depend on how many other
 // rows are in the call.
 //

@@ -5,8 +5,9 @@ one `Kernels` object the parts call into.  There is no other implementation: wit
 CUDA device of compute capability 10.x, or without a working build, `load()` raises.
 
 Every wrapper takes torch tensors that live on the GPU, checks dtype, shape and layout,
-and launches on torch's current stream.  Matrix products in float32 always run this
-library's FMA kernel.  In bfloat16 they run this library's tcgen05 kernels where those are
+and launches on torch's current stream.  Matrix products in float32 run this library's
+tensor-core kernel of bfloat16 pieces (csrc/gemm_f32_tc.cu; rows off a 16-byte boundary its FMA kernel), at
+float32 precision.  In bfloat16 they run this library's tcgen05 kernels where those are
 the faster ones (every product of a decode step of up to 32 tokens; the fused SwiGLU product
 up to 128 tokens and, on the CTA-pair kernel, from 640 tokens), else cuBLAS through torch
 (`torch.mm`), the library the reference's engine uses for them (engine/model.py:194,
@@ -73,6 +74,9 @@ _SIGNATURES = {
     "llm_attention_tcgen05_status": [],
     "llm_gemm_f32": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                      _c_void_p],
+    "llm_gemm_f32_tc_supported": [_c_int, _c_void_p, _c_void_p],
+    "llm_gemm_f32_tc_scratch": [_c_int, _c_int],
+    "llm_gemm_f32_tc": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
     "llm_gemm_bf16_token_tile": [_c_int],
     "llm_gemm_bf16": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p,
                       _c_int, _c_int, _c_int, _c_void_p],
@@ -394,6 +398,7 @@ class Kernels:
             fn = getattr(self.lib, name)
             fn.argtypes = args
             fn.restype = _c_int
+        self.lib.llm_gemm_f32_tc_scratch.restype = ctypes.c_longlong
         self.launches = 0  # kernels of this library launched so far (the bench reports it)
         # IITJ_GEMM_BACKEND=cublas|tcgen05 forces one matrix-product path, IITJ_GEMM_SMALL_TOKENS moves the
         # SwiGLU boundary, IITJ_PDL=0 switches programmatic dependent launch off (all for measurements)
@@ -1673,8 +1678,17 @@ class Kernels:
         if x.shape[0] == 0:
             return out
         if x.dtype == torch.float32:
-            self._call("llm_gemm_f32", _ptr(x), _ptr(weight), _ptr(out), x.shape[0], n, x.shape[1], x.shape[1],
-                       weight.shape[1], n, 1 if swiglu else 0, self._stream())
+            # which kernel depends on the row length alone (and on the alignment that TMA asks for), never on the token count:
+            # a row's product is the same whatever else is in the call
+            rows, k = x.shape
+            if self.lib.llm_gemm_f32_tc_supported(k, _ptr(x), _ptr(weight)):
+                # (from torch's caching allocator and not from the shared scratch: float32 products may run on several streams)
+                planes = torch.empty(self.lib.llm_gemm_f32_tc_scratch(rows, k), dtype=torch.bfloat16, device=x.device)
+                self._call("llm_gemm_f32_tc", _ptr(x), _ptr(weight), _ptr(out), rows, n, k, n, 1 if swiglu else 0, _ptr(planes),
+                           self._stream())
+                self.launches += 1
+            else:
+                self._call("llm_gemm_f32", _ptr(x), _ptr(weight), _ptr(out), rows, n, k, k, k, n, 1 if swiglu else 0, self._stream())
             return out
         # bfloat16: this library's tcgen05 kernel where it is the faster one, else cuBLAS through torch
         tokens, k = x.shape

@@ -1,0 +1,98 @@
+"""float32 products on the tensor cores (csrc/gemm_f32_tc.cu) against the same product in 64 bits.
+
+Bound: every factor is held exactly in three bfloat16 pieces; left out are piece products of at most 2^-23 of a product, and
+a chunk of 128 k is added up by the tensor cores in eight steps that cut off (at most 2^-23 of the running sum each), which
+shrinks a chunk by less than 8 * 2^-23 / 2 = 4.8e-7 of itself in the mean.  In the 2-norm of a result with random signs that and
+the rounded sum over at most 160 chunks stay below 1e-6."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def K():
+    from iitj_llm_coopt_b200 import kernels
+    return kernels.load()
+
+
+def product(x, w, swiglu=False):
+    y = x.double() @ w.double().t()
+    if swiglu:
+        n = w.shape[0] // 2
+        y = torch.nn.functional.silu(y[:, :n]) * y[:, n:]
+    return y
+
+
+def rnd(shape, seed, scale=1.0):
+    return torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda") * scale
+
+
+# token counts at the edges of the two kernels and of the tiles; k at one piece, at the edges of boxes (32), steps (64), chunks (128) and
+# segments (256), with every kind of cluster (2 .. 8 blocks) and beyond eight chunks a block
+@pytest.mark.parametrize("tokens", [1, 16, 17, 80, 81, 333])
+@pytest.mark.parametrize("n,k", [(1, 4), (130, 36), (128, 64), (129, 132), (64, 256), (200, 264), (300, 1028), (130, 1792), (257, 4104), (64, 20000)])
+def test_product(K, tokens, n, k):
+    for swiglu in (False, True):
+        x, w = rnd((tokens, k), 1), rnd(((2 if swiglu else 1) * n, k), 2, k ** -0.5)
+        out = torch.full((tokens + 1, n), 7.0, device="cuda")
+        K.linear(x, w, out[:tokens], swiglu=swiglu)
+        want = product(x, w, swiglu)
+        assert ((out[:tokens] - want).norm() / want.norm()).item() < 1e-6
+        assert (out[tokens] == 7.0).all() and K.gemm_status() == 0
+        row = torch.empty(1, n, device="cuda")                   # a row by itself: the same number, bit for bit
+        K.linear(x[tokens // 2:tokens // 2 + 1].contiguous(), w, row, swiglu=swiglu)
+        assert torch.equal(row[0], out[tokens // 2])
+
+
+# more blocks than the GPU holds at a time, so that loads land late and in any order: every kind of block, with and without clusters
+@pytest.mark.parametrize("tokens,n,k", [(5, 40000, 2048), (16, 9000, 8192), (200, 20000, 1024), (32, 6000, 4096)])
+def test_many_blocks(K, tokens, n, k):
+    x, w = rnd((tokens, k), 1), rnd((n, k), 2, k ** -0.5)
+    out = torch.empty(tokens, n, device="cuda")
+    K.linear(x, w, out)
+    want = product(x, w)
+    assert ((out - want).norm() / want.norm()).item() < 1e-6 and K.gemm_status() == 0
+
+
+def test_infinities_and_nans_go_where_they_would(K):
+    x, w = rnd((40, 300), 3), rnd((70, 300), 4)
+    x[3, 5], x[4, 299], x[5, 0] = float("inf"), float("nan"), -float("inf")
+    w[7, 5] = float("inf")
+    w[8, :] = 0.0
+    x[6, 11] = 3.4e38                                            # rounds to infinity in eight bits; stays finite here
+    w[:, 11] = w[:, 11].abs().clamp(1e-3, 0.9)
+    want = (x.double() @ w.double().t()).float()
+    for rows in (slice(0, 40), slice(0, 9)):
+        out = torch.empty(40, 70, device="cuda")[rows]
+        K.linear(x[rows].contiguous(), w, out)
+        assert torch.equal(out.isnan(), want[rows].isnan()) and torch.equal(out.isposinf(), want[rows].isposinf())
+        assert torch.equal(out.isneginf(), want[rows].isneginf())
+        ok = want[rows].isfinite()
+        assert ((out - want[rows])[ok].abs() <= 1e-5 * want[rows][ok].abs() + 1e-4).all()
+
+
+def test_rows_that_start_off_a_boundary_take_the_other_kernel(K):
+    base = rnd((5 * 64 + 1,), 5)
+    x, w = base[1:].view(5, 64), rnd((30, 64), 6)
+    assert not K.lib.llm_gemm_f32_tc_supported(64, x.data_ptr(), w.data_ptr()) and not K.lib.llm_gemm_f32_tc_supported(66, w.data_ptr(), w.data_ptr())
+    out = torch.empty(5, 30, device="cuda")
+    K.linear(x, w, out)
+    assert ((out - product(x, w)).norm() / product(x, w).norm()).item() < 1e-6
+
+
+def test_on_two_streams_at_once(K):
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    xs, ws = [rnd((100, 512), 7 + i) for i in range(2)], [rnd((700, 512), 9 + i) for i in range(2)]
+    want = [product(x, w) for x, w in zip(xs, ws)]
+    torch.cuda.synchronize()
+    outs = [[torch.empty(100, 700, device="cuda") for _ in range(20)] for _ in range(2)]
+    torch.cuda.synchronize()
+    for j in range(20):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                K.linear(xs[i], ws[i], outs[i][j])
+    torch.cuda.synchronize()
+    for i in range(2):
+        for o in outs[i]:
+            assert ((o - want[i]).norm() / want[i].norm()).item() < 1e-6
