@@ -1,8 +1,8 @@
 // Paged causal attention, general form: any head size that is a multiple of 16 up to 256,
 // any number of heads and groups, any page size, optional sliding window, float32 or
-// bfloat16 storage, float32 arithmetic throughout.  It is the whole of the float32 path
-// (prompt portions and decoded tokens alike) and the bfloat16 path's fallback for head
-// sizes that the tensor-core kernels do not take.
+// bfloat16 storage, float32 arithmetic throughout.  It serves the head sizes that neither
+// the float32 kernels (attention_f32.cu, the same sums bit for bit) nor the bfloat16
+// tensor-core kernels take.
 //
 // Replaces flash_attn_varlen_func with block_table (engine/model.py:204-207): a query at
 // position p of request b sees the keys at positions [lo, p] of that request, lo = 0 or

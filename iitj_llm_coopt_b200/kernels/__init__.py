@@ -50,6 +50,11 @@ _SIGNATURES = {
     "llm_sum_parts": [_c_void_p, _c_void_p, _c_int, _c_int, ctypes.c_longlong, _c_void_p],
     "llm_attention_generic": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p,
                               _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_void_p],
+    "llm_attention_f32_supported": [_c_int, _c_int, _c_int],
+    "llm_attention_f32_tiles": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int,
+                                _c_int, _c_int, _c_int, _c_float, _c_void_p],
+    "llm_attention_f32_single": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p,
+                                 _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_void_p],
     "llm_attention_bf16_supported": [_c_int, _c_int, _c_int],
     "llm_attention_prefill_bf16": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int,
                                    _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_void_p],
@@ -756,11 +761,30 @@ class Kernels:
                 if splits > 1:
                     self.launches += 1      # the merge kernel
             return out
+        if self._attention_f32_takes(qkv, cache_layer, meta, out, heads, kv_heads, head_dim):
+            plan = attention_plan(meta, qkv.device)
+            if max(plan.n_tiles, plan.n_items) <= 65535:
+                if plan.n_tiles:
+                    self._call("llm_attention_f32_tiles", _ptr(qkv), qkv.shape[1], _ptr(cache_layer), _ptr(meta.block_table),
+                               meta.block_table.shape[1], _ptr(plan.tiles), plan.n_tiles, _ptr(out), out.shape[1], heads, kv_heads,
+                               head_dim, page_size, int(window), float(scale), self._stream())
+                if plan.n_items:
+                    self._call("llm_attention_f32_single", _ptr(qkv), qkv.shape[1], _ptr(cache_layer), _ptr(meta.block_table),
+                               meta.block_table.shape[1], _ptr(plan.items), plan.n_items, _ptr(meta.token_request), _ptr(meta.positions),
+                               _ptr(out), out.shape[1], heads, kv_heads, head_dim, page_size, int(window), float(scale), self._stream())
+                return out
         self._call("llm_attention_generic", _ptr(qkv), qkv.shape[1], _ptr(cache_layer), _ptr(meta.block_table),
                    meta.block_table.shape[1], _ptr(meta.token_request), _ptr(meta.positions), _ptr(out),
                    out.shape[1], DTYPE_CODE[qkv.dtype], tokens, heads, kv_heads, head_dim, page_size,
                    int(window), float(scale), self._stream())
         return out
+
+    def _attention_f32_takes(self, qkv, cache_layer, meta, out, heads, kv_heads, head_dim) -> bool:
+        """True if float32 attention runs on the tile and single-token kernels: head sizes 64 and 128, rows on 16-byte
+        boundaries, and a `meta` that says how the tokens form requests.  They give the general kernel's numbers bit for bit."""
+        return bool(qkv.dtype == torch.float32 and qkv.shape[1] % 4 == 0 and getattr(meta, "query_lens", None) is not None and
+                    not (qkv.data_ptr() | out.data_ptr() | cache_layer.data_ptr()) & 15 and
+                    self.lib.llm_attention_f32_supported(heads, kv_heads, head_dim))
 
     def _decode_by_tma(self, cache_layer, heads, kv_heads, head_dim) -> bool:
         """True if decode attention fetches this cache layer's keys and values by TMA: a page size of 8 to 64 tokens, and
