@@ -16,21 +16,21 @@
 //
 // One block owns 128 rows of W (SwiGLU: 64 gate rows and the 64 up rows of the same features) and a tile of 16 to 80 tokens:
 //   loader      W in boxes of 32 k (128 bytes a row, 128-byte swizzle) by TMA, requested before the kernel ahead has finished
-//   converters  eight warps, a row a thread: 64 floats a step from shared memory, three pieces, into tensor memory as the A operand
+//   converters  two groups of four warps, a row a thread: 32 floats a step and group from shared memory, three pieces, into tensor memory as the A operand
 //               (the weights' pieces then cost the product no shared-memory bandwidth)
 //   x           split_planes_kernel lays the pieces out once and TMA loads them.  (Taking x apart in every block costs a proxy fence
 //               a step on top of the work: products of few tokens took 2300 clocks a step that way.)
-//   issuer      one warp: sixteen tcgen05.mma a step of 64 k
+//   issuers     two warps, one for the large and one for the small products: sixteen tcgen05.mma a step of 64 k
 //   epilogue    four or eight warps, a row a thread: chunks out of tensor memory, sums in registers
 // A step's barriers (a wait takes 200 clocks even when there is nothing to wait for, a commit 100) cost the issuer and the converters
-// about 1000 clocks whatever the tile, as much as the products of 80 tokens take: hence steps of 64 k and not fewer.
+// about 1000 clocks whatever the tile, as much as the products of 80 tokens take: hence steps of 64 k and not fewer, and two issuers.
 // Products with few tiles share the k range out over a cluster of blocks (segments whole): every block keeps the sums of its
 // chunks in shared memory, and the blocks then add all chunks of their part of the tile in order, over distributed shared memory.
 //
 // What bounds it: a decode step the HBM bytes of W, a prompt the tensor cores at six bfloat16 products per float32 product (278
 // TFLOP/s of the measured bf16 rate) and the barriers above.  Measured, cold weights, against the product on the CUDA cores
-// (gemm_f32.cu): 5 tokens, 2048 x 2048 195 -> 9 us, 2048 x 8192 770 -> 40 us, 128256 x 2048 1006 -> 180 us (5.8 TB/s);
-// 777 tokens, 2048 x 2048 256 -> 69 us, 2048 x 8192 993 -> 219 us (119 TFLOP/s), SwiGLU 8192 x 2048 1483 -> 419 us.
+// (gemm_f32.cu): 5 tokens, 2048 x 2048 195 -> 9 us, 2048 x 8192 770 -> 36 us, 128256 x 2048 1006 -> 173 us (6.1 TB/s);
+// 777 tokens, 2048 x 2048 256 -> 66 us, 2048 x 8192 993 -> 196 us (133 TFLOP/s), SwiGLU 8192 x 2048 1483 -> 331 us (157 TFLOP/s).
 //
 // Infinities and NaNs arrive through hi.hi as they would in a plain product; the small products, which then hold inf - inf, are left
 // out when they are not finite.  Waits are bounded: a wait that runs out records a code in the status word of the bfloat16 product
@@ -45,9 +45,9 @@ constexpr int kRows = 128;               // rows of W per block (UMMA M)
 constexpr int kStepK = 64;               // k of a step: two boxes of W of 32 float32 a row
 constexpr int kBoxBytes = kRows * 32 * 4;
 constexpr int kChunkSteps = 2;           // steps whose hi.hi products stay in one accumulator
-// Ring stages; of W: boxes, a multiple of four, so that a stage is always read by the same group of converters.  (Boxes land in any
+// Ring stages; of W: boxes, an even number, so that a stage is always read by the same group of converters.  (Boxes land in any
 // order: a group that shared a stage could come to wait for the stage's second box before the first, the other group's, had landed,
-// and a wait by parity that is two phases early passes at once.)  The A slots are an even number for the same reason.
+// and a wait by parity that is two phases early passes at once.)
 constexpr int kMaxW = 12, kMaxX = 4;
 constexpr int kACols = 96;               // tensor-memory columns of the A pieces of one step
 constexpr int kMaxA = 4;                 // steps whose A pieces lie in tensor memory at a time
@@ -68,9 +68,11 @@ struct Args {
 
 __device__ __forceinline__ void give_up_f32(const Args& a, int code) { atomicCAS(a.status, 0, (code << 16) | (int)(blockIdx.x & 0xffff)); }
 
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -140,15 +142,15 @@ __device__ __forceinline__ float silu_mul_f32(float g, float u) { return g / (1.
 template <bool SMALL>
 __global__ void __launch_bounds__(SMALL ? 512 : 640, SMALL ? 2 : 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Args a) {
-    constexpr int kEpiWarps = SMALL ? 4 : 8, kGroups = 2;       // groups of four converter warps
-    constexpr int kFirstEpi = 4 + 4 * kGroups;
+    constexpr int kEpiWarps = SMALL ? 4 : 8;
+    constexpr int kFirstEpi = 12;
     constexpr int kCols = SMALL ? 16 : 40;           // columns (tokens) of an epilogue thread
     extern __shared__ unsigned char smem_raw[];
     unsigned char* ring = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* xp = ring + a.ring_bytes;
     float* sums = reinterpret_cast<float*>(xp + a.x_bytes);
     __shared__ __align__(8) uint64_t w_full[kMaxW], w_empty[kMaxW], x_full[kMaxX], x_empty[kMaxX];
-    __shared__ __align__(8) uint64_t a_full[kMaxA], a_empty[kMaxA], chunk_full[2], hi_free[2], corr_free;
+    __shared__ __align__(8) uint64_t a_full[kMaxA], a_empty[kMaxA], chunk_full[2], hi_free[2], corr_full, corr_free;
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile int failed;
 
@@ -164,9 +166,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < a.w_stages; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 4); }
-        for (int s = 0; s < a.x_stages; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], 1); }
-        for (int s = 0; s < a.a_slots; ++s) { mbar_init(&a_full[s], 4); mbar_init(&a_empty[s], 1); }
+        for (int s = 0; s < a.x_stages; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], 2); }
+        for (int s = 0; s < a.a_slots; ++s) { mbar_init(&a_full[s], 8); mbar_init(&a_empty[s], 2); }
         for (int s = 0; s < 2; ++s) { mbar_init(&chunk_full[s], 1); mbar_init(&hi_free[s], kEpiWarps); }
+        mbar_init(&corr_full, 1);
         mbar_init(&corr_free, kEpiWarps);
         failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -182,36 +185,44 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const uint32_t t_hi = tmem, t_corr = tmem + 2 * a.tt, t_a = tmem + 4 * a.tt;
 
     pdl_trigger();
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // ---- loader of W: the weights depend on no earlier kernel ----------------------------------------------
-        auto load_w = [&](int b, int s) {
-            unsigned char* st = ring + (size_t)s * kBoxBytes;
-            mbar_expect_tx(&w_full[s], kBoxBytes);
-            const int k = step0 * kStepK + 32 * b;
-            tma_load_2d(st, &map_w, &w_full[s], k, feat0);
-            if (a.swiglu) tma_load_2d(st + kBoxBytes / 2, &map_w, &w_full[s], k, a.n + feat0);
-        };
-        const int boxes = 2 * n_steps, pre = boxes < a.w_stages ? boxes : a.w_stages;
-        for (int b = 0; b < pre; ++b) load_w(b, b);
-        uint32_t phase = 0;
-        for (int b = pre, s = 0; b < boxes; ++b) {
-            if (!mbar_wait(&w_empty[s], phase)) { give_up_f32(a, 1); failed = 1; break; }
-            load_w(b, s);
+        const int boxes = 2 * n_steps, k_first = step0 * kStepK;
+        uint32_t phase = 1;
+        bool free_now = true;                          // what a poll after the box before has found
+        for (int b = 0, s = 0; b < boxes; ++b) {
+            if (b >= a.w_stages && !free_now && !mbar_wait(&w_empty[s], phase)) { if (lane == 0) give_up_f32(a, 1); failed = 1; break; }
+            if (elect_one()) {
+                unsigned char* st = ring + (size_t)s * kBoxBytes;
+                mbar_expect_tx(&w_full[s], kBoxBytes);
+                tma_load_2d(st, &map_w, &w_full[s], k_first + 32 * b, feat0);
+                if (a.swiglu) tma_load_2d(st + kBoxBytes / 2, &map_w, &w_full[s], k_first + 32 * b, a.n + feat0);
+            }
+            __syncwarp();
             if (++s == a.w_stages) { s = 0; phase ^= 1; }
+            if (b + 1 >= a.w_stages) {
+                const bool now = mbar_poll(&w_empty[s], phase);
+                free_now = __all_sync(0xffffffffu, now);
+            }
         }
-    } else if (warp == 2 && lane == 0) {
+    } else if (warp == 2) {
         // ---- loader of x's pieces: three boxes of 64 k ----------------------------------------------------------
         pdl_wait();
         uint32_t phase = 1;
         for (int j = 0, s = 0; j < n_steps; ++j) {
-            if (j >= a.x_stages && !mbar_wait(&x_empty[s], phase)) { give_up_f32(a, 1); failed = 1; break; }
-            mbar_expect_tx(&x_full[s], x_stage);
-            for (int p = 0; p < 3; ++p)
-                tma_load_2d(xp + (size_t)s * x_stage + p * a.tt * 128, &map_x, &x_full[s], (step0 + j) * kStepK, p * a.tokens + tok0);
+            if (j >= a.x_stages && !mbar_wait(&x_empty[s], phase)) { if (lane == 0) give_up_f32(a, 1); failed = 1; break; }
+            if (elect_one()) {
+                mbar_expect_tx(&x_full[s], x_stage);
+#pragma unroll
+                for (int p = 0; p < 3; ++p)
+                    tma_load_2d(xp + (size_t)s * x_stage + p * a.tt * 128, &map_x, &x_full[s], (step0 + j) * kStepK, p * a.tokens + tok0);
+            }
+            __syncwarp();
             if (++s == a.x_stages) { s = 0; phase ^= 1; }
         }
-    } else if (warp == 1) {
-        // ---- issuer (counters run along: a division costs it 100 clocks) -----------------------------------------
+    } else if (warp == 1 || warp == 3) {
+        // ---- issuers: warp 1 of the large products, warp 3 of the small ones (counters run along: a division costs them 100 clocks) --
+        const bool large = warp == 1;
         const uint32_t idesc1 = umma_idesc(kRows, a.tt), idesc2 = umma_idesc(kRows, 2 * a.tt);
         const uint64_t plane = (uint64_t)(a.tt * 128) >> 4, desc0 = umma_desc(xp), desc_stage = (uint64_t)x_stage >> 4;
         uint64_t desc = desc0;
@@ -222,27 +233,35 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             const int c = i / kChunkSteps;
             const bool seg_start = seg_left == a.seg_steps, chunk_start = i % kChunkSteps == 0;
             bool ok = x_ok || mbar_wait(&x_full[xs], x_phase);
-            if (chunk_start && c >= 2) ok = ok && (hi_ok || mbar_wait(&hi_free[c & 1], ((c / 2) - 1) & 1));
-            if (seg_start && i > 0) ok = ok && mbar_wait(&corr_free, (seg++) & 1);
+            if (large && chunk_start && c >= 2) ok = ok && (hi_ok || mbar_wait(&hi_free[c & 1], ((c / 2) - 1) & 1));
+            if (!large && seg_start && i > 0) ok = ok && mbar_wait(&corr_free, (seg++) & 1);
             ok = ok && (a_ok || mbar_wait(&a_full[as], a_phase));
             if (!ok) { if (lane == 0) give_up_f32(a, 2); failed = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t a0 = t_a + as * kACols, d_hi = t_hi + (c & 1) * a.tt;
-            // the pieces of x lie one after the other, so that one instruction multiplies a piece of W with two of them:
-            // the small products of order 2^-8 add up in one half of t_corr, those of order 2^-16 in the other
+            const bool last = i == n_steps - 1;
             if (elect_one()) {
+                if (large) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const uint32_t ah = a0 + 8 * k, am = ah + 32, al = ah + 64;
-                    const uint64_t bh = desc + 2 * k, bm = bh + plane;
-                    umma_ts(d_hi, ah, bh, idesc1, !(chunk_start && k == 0));
-                    umma_ts(t_corr, ah, bm, idesc2, !(seg_start && k == 0));          // hi.mid | hi.lo
-                    umma_ts(t_corr, am, bh, idesc2, 1u);                              // mid.hi | mid.mid
-                    umma_ts(t_corr + a.tt, al, bh, idesc1, 1u);                       //        | lo.hi
+                    for (int k = 0; k < 4; ++k) umma_ts(d_hi, a0 + 8 * k, desc + 2 * k, idesc1, !(chunk_start && k == 0));
+                    umma_commit(&a_empty[as]);
+                    umma_commit(&x_empty[xs]);
+                    if (i % kChunkSteps == kChunkSteps - 1 || last) umma_commit(&chunk_full[c & 1]);
+                } else {
+                    // the pieces of x lie one after the other, so that one instruction multiplies a piece of W with two of them:
+                    // the small products of order 2^-8 add up in one half of t_corr, those of order 2^-16 in the other
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const uint32_t ah = a0 + 8 * k, am = ah + 32, al = ah + 64;
+                        const uint64_t bh = desc + 2 * k, bm = bh + plane;
+                        umma_ts(t_corr, ah, bm, idesc2, !(seg_start && k == 0));          // hi.mid | hi.lo
+                        umma_ts(t_corr, am, bh, idesc2, 1u);                              // mid.hi | mid.mid
+                        umma_ts(t_corr + a.tt, al, bh, idesc1, 1u);                       //        | lo.hi
+                    }
+                    umma_commit(&a_empty[as]);
+                    umma_commit(&x_empty[xs]);
+                    if (seg_left == 1 || last) umma_commit(&corr_full);
                 }
-                umma_commit(&a_empty[as]);
-                umma_commit(&x_empty[xs]);
-                if (i % kChunkSteps == kChunkSteps - 1 || i == n_steps - 1) umma_commit(&chunk_full[c & 1]);
             }
             __syncwarp();
             desc += desc_stage;
@@ -251,51 +270,42 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             if (--seg_left == 0) seg_left = a.seg_steps;
             const int cn = (i + 1) / kChunkSteps;
             const bool x_now = mbar_poll(&x_full[xs], x_phase), a_now = mbar_poll(&a_full[as], a_phase);
-            const bool hi_now = cn >= 2 && mbar_poll(&hi_free[cn & 1], ((cn / 2) - 1) & 1);
+            const bool hi_now = large && cn >= 2 && mbar_poll(&hi_free[cn & 1], ((cn / 2) - 1) & 1);
             x_ok = __all_sync(0xffffffffu, x_now); a_ok = __all_sync(0xffffffffu, a_now); hi_ok = __all_sync(0xffffffffu, hi_now);
         }
     } else if (warp >= 4 && warp < kFirstEpi) {
-        // ---- converters: W's pieces into tensor memory, a group of four warps every kGroups-th step ---------------
+        // ---- converters: W's pieces into tensor memory; each group of four warps has one of the two boxes of every step ------------
         const int q = warp & 3, group = (warp - 4) >> 2, row = q * 32 + lane, sw = row & 7;
         uint32_t phase = 0, a_phase = 1;
-        int s = 0, as = group;
-        auto advance = [&](int by) { for (s += by; s >= a.w_stages; s -= a.w_stages) phase ^= 1; };
-        if (group) advance(2);
-        for (int i = group; i < n_steps; i += kGroups) {
-            const uint32_t ta = t_a + as * kACols + ((uint32_t)(q * 32) << 16);
-            bool ok = true;
+        bool w_ok = false;                                     // what a poll during the step before has found
+        for (int i = 0, s = group, as = 0; i < n_steps; ++i) {
+            if (!w_ok && !mbar_wait(&w_full[s], phase)) { if (lane == 0) give_up_f32(a, 4); failed = 1; break; }
+            const unsigned char* st = ring + (size_t)s * kBoxBytes + row * 128;
+            // the whole box is taken apart before the wait for the slot, so that only the stores lie between a slot's last product and
+            // its next one
+            const bool a_now = i < a.a_slots || mbar_poll(&a_empty[as], a_phase);
+            uint32_t hi[16], mid[16], lo[16];
 #pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                ok = ok && mbar_wait(&w_full[s], phase);
-                const unsigned char* st = ring + (size_t)s * kBoxBytes + row * 128;
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    uint32_t hi[8], mid[8], lo[8];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float4 v = *reinterpret_cast<const float4*>(st + (((4 * u + j) ^ sw) << 4));
-                        split2(v.x, v.y, hi[2 * j], mid[2 * j], lo[2 * j]);
-                        split2(v.z, v.w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
-                    }
-                    if (b == 0 && u == 0) {
-                        if (i >= a.a_slots) ok = ok && mbar_wait(&a_empty[as], a_phase);
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    }
-                    tmem_st8(ta + 16 * b + 8 * u, hi);
-                    tmem_st8(ta + 32 + 16 * b + 8 * u, mid);
-                    tmem_st8(ta + 64 + 16 * b + 8 * u, lo);
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&w_empty[s]);            // the box has been read
-                advance(1);
+            for (int j = 0; j < 8; ++j) {
+                const float4 v = *reinterpret_cast<const float4*>(st + ((j ^ sw) << 4));
+                split2(v.x, v.y, hi[2 * j], mid[2 * j], lo[2 * j]);
+                split2(v.z, v.w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
             }
-            if (!ok) { if (lane == 0) give_up_f32(a, 4); failed = 1; break; }
+            const bool a_ok = __all_sync(0xffffffffu, a_now);
+            if (lane == 0) mbar_arrive(&w_empty[s]);            // the box has been read
+            if ((s += 2) >= a.w_stages) { s -= a.w_stages; phase ^= 1; }
+            const bool w_now = mbar_poll(&w_full[s], phase);
+            if (!a_ok && !mbar_wait(&a_empty[as], a_phase)) { if (lane == 0) give_up_f32(a, 4); failed = 1; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t ta = t_a + as * kACols + 16 * group + ((uint32_t)(q * 32) << 16);
+            tmem_st16(ta, hi);
+            tmem_st16(ta + 32, mid);
+            tmem_st16(ta + 64, lo);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
+            w_ok = __all_sync(0xffffffffu, w_now);
             if (lane == 0) mbar_arrive(&a_full[as]);
-            if (kGroups > 1) advance(2);
-            if ((as += kGroups) >= a.a_slots) { as -= a.a_slots; a_phase ^= 1; }
+            if (++as == a.a_slots) { as = 0; a_phase ^= 1; }
         }
     } else if (warp >= kFirstEpi) {
         // ---- epilogue: chunks out of tensor memory ----------------------------------------------------------------
@@ -305,11 +315,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
         for (int j = 0; j < kCols; ++j) total[j] = 0.f;
         bool ok = true;
-        int seg_left = a.seg_steps / kChunkSteps;
+        int seg_left = a.seg_steps / kChunkSteps, seg = 0;
         for (int c = 0; c < n_chunks; ++c) {
             const bool seg_end = --seg_left == 0 || c == n_chunks - 1;
             if (seg_left == 0) seg_left = a.seg_steps / kChunkSteps;
-            if (!mbar_wait(&chunk_full[c & 1], (c / 2) & 1)) { if (lane == 0) give_up_f32(a, 3); failed = 1; ok = false; break; }
+            if (!mbar_wait(&chunk_full[c & 1], (c / 2) & 1) || (seg_end && !mbar_wait(&corr_full, (seg++) & 1))) { if (lane == 0) give_up_f32(a, 3); failed = 1; ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
             for (int g = 0; g < kCols; g += 8) {
@@ -343,22 +353,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if (a.cluster == 1) {
             pdl_wait();                                    // nothing is stored before the previous kernel has finished
             if (a.swiglu) {
-                // rows 64 .. 127 are up rows: handed to the threads of the gate rows through the ring, which has been read
-                float* up = reinterpret_cast<float*>(ring);
-                if (ok && q >= 2) {
+                // rows 0 .. 63 are gate rows, 64 .. 127 the up rows of the same features: through the ring, which has been read, to
+                // all threads of the block (below)
+                float* rows = reinterpret_cast<float*>(ring);
 #pragma unroll
-                    for (int j = 0; j < kCols; ++j)
-                        if (col0 + j < a.tt) up[(size_t)(col0 + j) * 64 + row - 64] = total[j];
-                }
-                asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-                if (ok && q < 2 && feat0 + row < a.n) {
-#pragma unroll
-                    for (int j = 0; j < kCols; ++j) {
-                        const int tok = tok0 + col0 + j;
-                        if (col0 + j < a.tt && tok < a.tokens)
-                            a.out[(size_t)tok * a.ldc + feat0 + row] = silu_mul_f32(total[j], up[(size_t)(col0 + j) * 64 + row]);
-                    }
-                }
+                for (int j = 0; j < kCols; ++j)
+                    if (ok && col0 + j < a.tt) rows[(size_t)(col0 + j) * kRows + row] = total[j];
             } else if (ok && feat0 + row < a.n) {
 #pragma unroll
                 for (int j = 0; j < kCols; ++j) {
@@ -370,6 +370,17 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (a.cluster == 1 && a.swiglu && !failed) {
+        pdl_wait();
+        const float* rows = reinterpret_cast<const float*>(ring);
+        const int live = min(a.tt, a.tokens - tok0);
+#pragma unroll 4
+        for (int e = threadIdx.x; e < live * 64; e += blockDim.x) {
+            const int col = e >> 6, row = e & 63;
+            if (feat0 + row < a.n)
+                a.out[(size_t)(tok0 + col) * a.ldc + feat0 + row] = silu_mul_f32(rows[col * kRows + row], rows[col * kRows + 64 + row]);
+        }
+    }
     if (a.cluster > 1) {
         __syncwarp();
         llm_cluster_sync();                                // every block's chunk sums lie in its shared memory
@@ -442,7 +453,7 @@ Plan make_plan(int tokens, int n, int swiglu, int steps, int seg_steps, int sms)
             // two blocks an SM where their sums leave the rings room
             bool two = small && 4 * tt + 2 * kACols <= 256;
             auto w_stages = [&](int xs) {
-                const int room = ((two ? 112 * 1024 : kSmemLimit) - 1024 - sums - xs * x_stage) / kBoxBytes / 4 * 4;
+                const int room = ((two ? 112 * 1024 : kSmemLimit) - 1024 - sums - xs * x_stage) / kBoxBytes / 2 * 2;
                 return room < kMaxW ? room : kMaxW;
             };
             if (two && w_stages(2) < 4) two = false;
@@ -457,7 +468,7 @@ Plan make_plan(int tokens, int n, int swiglu, int steps, int seg_steps, int sms)
                                 (cl > 1 ? 2000.0 + 40.0 * chunks * cl * tt / 16 : 0.0);
             if (cost < best_cost) {
                 best_cost = cost;
-                const int cols = two || 4 * tt + 2 * kACols <= 256 ? 256 : 512, slots = (cols - 4 * tt) / kACols / 2 * 2;
+                const int cols = two || 4 * tt + 2 * kACols <= 256 ? 256 : 512, slots = (cols - 4 * tt) / kACols;
                 best = Plan{tt, cl, ws, xs, slots < kMaxA ? slots : kMaxA, cols, ws * kBoxBytes + xs * x_stage + sums + 1024};
             }
         }
