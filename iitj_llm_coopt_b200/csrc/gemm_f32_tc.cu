@@ -32,10 +32,15 @@
 // (gemm_f32.cu): 5 tokens, 2048 x 2048 195 -> 9 us, 2048 x 8192 770 -> 36 us, 128256 x 2048 1006 -> 173 us (6.1 TB/s);
 // 777 tokens, 2048 x 2048 256 -> 66 us, 2048 x 8192 993 -> 196 us (133 TFLOP/s), SwiGLU 8192 x 2048 1483 -> 331 us (157 TFLOP/s).
 //
+// Listed form (llm_gemm_f32_tc_listed): the rows were sorted by weight matrix on the device (the experts of a routed feed-forward);
+// a block takes its tile from the list, blocks beyond the list's count leave at once.
+//
 // Infinities and NaNs arrive through hi.hi as they would in a plain product; the small products, which then hold inf - inf, are left
 // out when they are not finite.  Waits are bounded: a wait that runs out records a code in the status word of the bfloat16 product
 // (1 producer, 2 issuer, 3 epilogue, 4 converter), and the block falls through to its teardown.
 #include "tcgen05_common.cuh"
+
+LLM_API int llm_gemm_grouped_tile_rows();      // gemm_grouped.cu
 
 namespace {
 
@@ -52,12 +57,18 @@ constexpr int kMaxW = 12, kMaxX = 4;
 constexpr int kACols = 96;               // tensor-memory columns of the A pieces of one step
 constexpr int kMaxA = 4;                 // steps whose A pieces lie in tensor memory at a time
 constexpr int kSmallTokens = 16;         // up to here the smaller kernel
+constexpr int kListedRows = 64;          // rows of a listed tile, at most (gemm_grouped.cu)
 constexpr int kMaxTile = 80;             // tokens of a tile: 4 x 80 accumulator columns and two slots of A fill tensor memory
 
 struct Args {
     float* out;
     int* status;
-    int n, ldc, tokens, swiglu;
+    int n, ldc, tokens, swiglu;          // swiglu: W holds gate rows, then up rows
+    // listed form (tiles != null): rows sorted by group beforehand, a weight matrix each (llm_moe_plan writes the list)
+    const int* tiles;                    // tiles[0] = count, entry i at tiles[4 + 4 * i] = (group, first row, rows, -)
+    int clamped;                         // the gate's form: 0 silu(w g) * (w u), 1 clamped
+    float limit, slope;
+    const float* row_scale;              // w of form 0, one per row (null: 1)
     int steps, seg_steps, segs;          // steps of 64 k; steps of a segment (a multiple of 2); segments
     int cluster;                         // blocks that share a tile's k range (a divisor of segs)
     int tt, t_tiles;                     // tokens of a tile (a multiple of 16); token tiles
@@ -135,7 +146,17 @@ __device__ __forceinline__ float cluster_sum(const float* p, int stride, int cou
     return t;
 }
 
-__device__ __forceinline__ float silu_mul_f32(float g, float u) { return g / (1.0f + expf(-g)) * u; }
+// What becomes of a gate and an up number of result row `r` (gemm_grouped.cu's two forms; a plain SwiGLU is form 0 with w = 1).
+__device__ __forceinline__ float glu(const Args& a, float g, float u, int r) {
+    if (a.clamped) {
+        g = fminf(g, a.limit);
+        u = fminf(fmaxf(u, -a.limit), a.limit);
+        return g / (1.0f + expf(-a.slope * g)) * (u + 1.0f);
+    }
+    const float w = a.row_scale ? a.row_scale[r] : 1.0f;
+    g *= w;
+    return g / (1.0f + expf(-g)) * (u * w);
+}
 
 // SMALL: one tile of at most 16 tokens; fewer threads of fewer registers, so that two blocks share an SM and the next product's
 // blocks can start on their weights while this one's finish.
@@ -157,8 +178,18 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int rank = a.cluster > 1 ? (int)llm_cluster_rank() : 0;
     // the token tiles of a block of W's rows are neighbours in the grid, so that W comes from HBM once
-    const int tile = blockIdx.x / a.cluster, tok0 = (tile % a.t_tiles) * a.tt;
+    const int tile = blockIdx.x / a.cluster;
     const int feat0 = (tile / a.t_tiles) * (a.swiglu ? kRows / 2 : kRows);
+    int tok0 = (tile % a.t_tiles) * a.tt, tok_end = min(a.tokens, tok0 + a.tt), w_row0 = feat0;
+    if (a.tiles) {
+        pdl_wait();                                    // the list is an earlier kernel's
+        const int i = tile % a.t_tiles;
+        if (i >= a.tiles[0]) return;                   // the whole cluster
+        const int* e = a.tiles + 4 + 4 * i;
+        tok0 = e[1];
+        tok_end = tok0 + min(e[2], a.tt);
+        w_row0 = e[0] * a.n * (a.swiglu ? 2 : 1) + feat0;
+    }
     const int block_steps = a.segs / a.cluster * a.seg_steps;
     const int step0 = rank * block_steps, n_steps = min(a.steps - step0, block_steps);
     const int n_chunks = (n_steps + kChunkSteps - 1) / kChunkSteps;
@@ -195,8 +226,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             if (elect_one()) {
                 unsigned char* st = ring + (size_t)s * kBoxBytes;
                 mbar_expect_tx(&w_full[s], kBoxBytes);
-                tma_load_2d(st, &map_w, &w_full[s], k_first + 32 * b, feat0);
-                if (a.swiglu) tma_load_2d(st + kBoxBytes / 2, &map_w, &w_full[s], k_first + 32 * b, a.n + feat0);
+                tma_load_2d(st, &map_w, &w_full[s], k_first + 32 * b, w_row0);
+                if (a.swiglu) tma_load_2d(st + kBoxBytes / 2, &map_w, &w_full[s], k_first + 32 * b, a.n + w_row0);
             }
             __syncwarp();
             if (++s == a.w_stages) { s = 0; phase ^= 1; }
@@ -363,7 +394,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
                 for (int j = 0; j < kCols; ++j) {
                     const int tok = tok0 + col0 + j;
-                    if (col0 + j < a.tt && tok < a.tokens) a.out[(size_t)tok * a.ldc + feat0 + row] = total[j];
+                    if (tok < tok_end) a.out[(size_t)tok * a.ldc + feat0 + row] = total[j];
                 }
             }
         }
@@ -373,19 +404,19 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     if (a.cluster == 1 && a.swiglu && !failed) {
         pdl_wait();
         const float* rows = reinterpret_cast<const float*>(ring);
-        const int live = min(a.tt, a.tokens - tok0);
+        const int live = tok_end - tok0;
 #pragma unroll 4
         for (int e = threadIdx.x; e < live * 64; e += blockDim.x) {
             const int col = e >> 6, row = e & 63;
             if (feat0 + row < a.n)
-                a.out[(size_t)(tok0 + col) * a.ldc + feat0 + row] = silu_mul_f32(rows[col * kRows + row], rows[col * kRows + 64 + row]);
+                a.out[(size_t)(tok0 + col) * a.ldc + feat0 + row] = glu(a, rows[col * kRows + row], rows[col * kRows + 64 + row], tok0 + col);
         }
     }
     if (a.cluster > 1) {
         __syncwarp();
         llm_cluster_sync();                                // every block's chunk sums lie in its shared memory
         pdl_wait();
-        const int rows = a.swiglu ? kRows / 2 : kRows, live = min(a.tt, a.tokens - tok0);
+        const int rows = a.swiglu ? kRows / 2 : kRows, live = tok_end - tok0;
         const int all_chunks = (a.steps + kChunkSteps - 1) / kChunkSteps;
         const int per_block = a.segs / a.cluster * (a.seg_steps / kChunkSteps);         // (the last block may have fewer)
         const int l = (threadIdx.x >> 3) & 3, per_pass = blockDim.x / 4, stride = a.tt * kRows;
@@ -396,7 +427,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             const float g = cluster_sum(p, stride, all_chunks, per_block, l);
             const float u = a.swiglu ? cluster_sum(p + kRows / 2, stride, all_chunks, per_block, l) : 0.f;
             if (l == 3 && e < live * rows && feat0 + row < a.n)
-                a.out[(size_t)(tok0 + col) * a.ldc + feat0 + row] = a.swiglu ? silu_mul_f32(g, u) : g;
+                a.out[(size_t)(tok0 + col) * a.ldc + feat0 + row] = a.swiglu ? glu(a, g, u, tok0 + col) : g;
         }
         __syncwarp();
         llm_cluster_sync();                                // nobody leaves while its shared memory is being read
@@ -407,17 +438,19 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
 }
 
-// planes[p][t][k], p = hi, mid, lo: the bfloat16 pieces of x, four numbers a thread; columns K .. kp - 1 are zero.
+// planes[p][t][k], p = hi, mid, lo: the bfloat16 pieces of x, four numbers a thread; columns K .. kp - 1 are zero.  Listed form: of
+// the first live_rows[0] rows alone, row t being row source[t] of x (null: t).
 __global__ void __launch_bounds__(256)
-split_planes_kernel(const float* __restrict__ x, bf16* __restrict__ planes, int tokens, int K, int kp) {
+split_planes_kernel(const float* __restrict__ x, bf16* __restrict__ planes, int tokens, int K, int kp, const int* __restrict__ source,
+                    const int* __restrict__ live_rows) {
     pdl_trigger();
     pdl_wait();
-    const int quads = kp / 4;
+    const int quads = kp / 4, live = live_rows ? min(tokens, live_rows[0]) : tokens;
     const size_t plane = (size_t)tokens * kp;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)tokens * quads; i += (size_t)gridDim.x * blockDim.x) {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)live * quads; i += (size_t)gridDim.x * blockDim.x) {
         const int t = (int)(i / quads), k = (int)(i % quads) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (k < K) v = *reinterpret_cast<const float4*>(x + (size_t)t * K + k);
+        if (k < K) v = *reinterpret_cast<const float4*>(x + (size_t)(source ? source[t] : t) * K + k);
         uint2 h, m, l;
         split2(v.x, v.y, h.x, m.x, l.x);
         split2(v.z, v.w, h.y, m.y, l.y);
@@ -435,18 +468,18 @@ struct Plan { int tt, cluster, w_stages, x_stages, a_slots, tmem_cols, smem; };
 // The cut of a product into tiles of `tt` tokens and clusters over the k range: the one with the least estimated clocks.  A step of
 // 64 k costs a block the larger of its tensor-core time (12 clocks a token) and its shared-memory time (64 KiB of W written and
 // read, 1152 bytes a token, at 128 bytes a clock), and about 1000 clocks of barriers whatever its size; blocks that share an SM share
-// the former two.
-Plan make_plan(int tokens, int n, int swiglu, int steps, int seg_steps, int sms) {
+// the former two.  Listed form: `listed` tiles are expected, of `tokens` rows at most.
+Plan make_plan(int tokens, int n, int swiglu, int steps, int seg_steps, int sms, int listed) {
     const int segs = (steps + seg_steps - 1) / seg_steps;
     const bool small = tokens <= kSmallTokens;
     const long long f_tiles = swiglu ? (n + 63) / 64 : (n + kRows - 1) / kRows;
     Plan best{};
     double best_cost = 1e30;
     const int most = tokens >= kMaxTile ? kMaxTile : (tokens + 15) / 16 * 16;
-    for (int tt = small ? most : 16; tt <= most; tt += 16)
+    for (int tt = small || listed ? most : 16; tt <= most; tt += 16)
         for (int cl = 1; cl <= segs; ++cl) {
             if (segs % cl) continue;
-            const long long ctas = f_tiles * ((tokens + tt - 1) / tt) * cl;
+            const long long ctas = f_tiles * (listed ? listed : (tokens + tt - 1) / tt) * cl;
             const int cta_steps = segs / cl * seg_steps < steps ? segs / cl * seg_steps : steps;
             const int chunks = (cta_steps + kChunkSteps - 1) / kChunkSteps;
             const int sums = cl > 1 ? chunks * tt * kRows * 4 : 0, x_stage = 3 * tt * 128;
@@ -498,42 +531,70 @@ LLM_API int llm_gemm_f32_tc_supported(int K, const void* x, const void* w) {
 // bfloat16 elements of scratch that a call with `tokens` rows needs.
 LLM_API long long llm_gemm_f32_tc_scratch(int tokens, int K) { return 3LL * tokens * ((K + 7) / 8 * 8); }
 
-// out [tokens, ldc] = x [tokens, K] . w [n, K]^T, or with swiglu silu(x . w[0:n]^T) * (x . w[n:2n]^T); rows of x and w contiguous.
-LLM_API int llm_gemm_f32_tc(const float* x, const float* w, float* out, int tokens, int n, int K, int ldc, int swiglu,
-                            void* planes, cudaStream_t stream) {
-    if (tokens == 0 || n == 0) return 0;
+namespace {
+
+// `tokens`: rows of x's pieces (and of the result); `groups` weight matrices; listed form: max_tiles > 0.
+int run(const float* x, const int* source, const float* w, int tokens, int groups, int max_tiles, int K, void* planes, Args a, cudaStream_t stream) {
     if (!llm_gemm_f32_tc_supported(K, x, w)) LLM_FAIL(-1, "gemm_f32_tc: rows of %d floats do not start on 16-byte boundaries", K);
     if (!planes || ((uintptr_t)planes & 15)) LLM_FAIL(-1, "gemm_f32_tc: scratch for the pieces of x, on a 16-byte boundary, is needed");
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         LLM_FAIL(-2, "gemm_f32_tc: no device");
-    Args a;
-    a.out = out; a.n = n; a.ldc = ldc; a.tokens = tokens; a.swiglu = swiglu ? 1 : 0;
+    a.tokens = tokens;
     a.status = const_cast<int*>(llm_gemm_bf16_status_word());
     if (!a.status) LLM_FAIL(-2, "gemm_f32_tc: no status word");
     a.steps = (K + kStepK - 1) / kStepK;
     a.seg_steps = ((a.steps + 7) / 8 + 1) / 2 * 2;
     if (a.seg_steps < 4) a.seg_steps = 4;
     a.segs = (a.steps + a.seg_steps - 1) / a.seg_steps;
-    const Plan p = make_plan(tokens, n, a.swiglu, a.steps, a.seg_steps, sms);
-    if (!p.tt) LLM_FAIL(-1, "gemm_f32_tc: no cut of %d x %d x %d fits", tokens, n, K);
+    const int tile_tokens = max_tiles && tokens > kListedRows ? kListedRows : tokens;
+    const Plan p = make_plan(tile_tokens, a.n, a.swiglu, a.steps, a.seg_steps, sms, max_tiles < tokens ? max_tiles : tokens);
+    if (!p.tt) LLM_FAIL(-1, "gemm_f32_tc: no cut of %d x %d x %d fits", tokens, a.n, K);
     a.cluster = p.cluster; a.tt = p.tt; a.w_stages = p.w_stages; a.x_stages = p.x_stages; a.a_slots = p.a_slots;
     a.ring_bytes = p.w_stages * kBoxBytes;
     a.x_bytes = p.x_stages * 3 * p.tt * 128;
     a.tmem_cols = p.tmem_cols;
-    a.t_tiles = (tokens + p.tt - 1) / p.tt;
-    const long long blocks_x = (long long)(swiglu ? (n + 63) / 64 : (n + kRows - 1) / kRows) * a.t_tiles * p.cluster;
-    if (blocks_x > 0x7fffffffLL) LLM_FAIL(-1, "gemm_f32_tc: %d tokens by %d are too many for one launch", tokens, n);
+    a.t_tiles = max_tiles ? max_tiles : (tokens + p.tt - 1) / p.tt;
+    const long long blocks_x = (long long)(a.swiglu ? (a.n + 63) / 64 : (a.n + kRows - 1) / kRows) * a.t_tiles * p.cluster;
+    if (blocks_x > 0x7fffffffLL) LLM_FAIL(-1, "gemm_f32_tc: %d tokens by %d are too many for one launch", tokens, a.n);
     const dim3 grid((unsigned)blocks_x);
     const int kp = (K + 7) / 8 * 8;
     CUtensorMap mw, mx;
-    if (int rc = llm_tensor_map_2d_f32(w, (uint64_t)n * (swiglu ? 2 : 1), K, swiglu ? kRows / 2 : kRows, 32, &mw)) return rc;
+    if (int rc = llm_tensor_map_2d_f32(w, (uint64_t)groups * a.n * (a.swiglu ? 2 : 1), K, a.swiglu ? kRows / 2 : kRows, 32, &mw)) return rc;
     if (int rc = llm_tensor_map_2d(planes, 3ull * tokens, kp, p.tt, 64, &mx)) return rc;
     const size_t quads = (size_t)tokens * (kp / 4);
     const int blocks = (int)((quads + 255) / 256 < 148 * 8 ? (quads + 255) / 256 : 148 * 8);
-    llm_launch(split_planes_kernel, blocks, 256, 0, stream, x, (bf16*)planes, tokens, K, kp);
+    llm_launch(split_planes_kernel, blocks, 256, 0, stream, x, (bf16*)planes, tokens, K, kp, source, a.tiles ? a.tiles + 1 : nullptr);
     LLM_CHECK_LAUNCH("gemm_f32_tc_planes");
-    return tokens <= kSmallTokens ? launch<true>(mw, mx, a, grid, p.smem, stream) : launch<false>(mw, mx, a, grid, p.smem, stream);
+    return tile_tokens <= kSmallTokens ? launch<true>(mw, mx, a, grid, p.smem, stream) : launch<false>(mw, mx, a, grid, p.smem, stream);
+}
+
+}  // namespace
+
+// out [tokens, ldc] = x [tokens, K] . w [n, K]^T, or with swiglu silu(x . w[0:n]^T) * (x . w[n:2n]^T); rows of x and w contiguous.
+LLM_API int llm_gemm_f32_tc(const float* x, const float* w, float* out, int tokens, int n, int K, int ldc, int swiglu,
+                            void* planes, cudaStream_t stream) {
+    if (tokens == 0 || n == 0) return 0;
+    Args a{};
+    a.out = out; a.n = n; a.ldc = ldc; a.swiglu = swiglu ? 1 : 0;
+    return run(x, nullptr, w, tokens, 1, 0, K, planes, a, stream);
+}
+
+// The listed form of llm_gemm_grouped: out [rows, ldc] = row r of x (row source[r], null: r) . w[group of r]^T for the rows that the
+// device's list of tiles names (of llm_gemm_grouped_tile_rows rows at most; tiles[1]: how many rows are live), with that entry's glu
+// forms (0 none, 1 clamped, 2 silu with a factor per row).  w [groups, n (2n with glu), K].
+LLM_API int llm_gemm_f32_tc_listed(const float* x, const int* source, const float* w, float* out, int rows, int n, int K, int groups,
+                                   const int* tiles, int max_tiles, int form, float limit, float slope, const float* row_scale,
+                                   void* planes, cudaStream_t stream) {
+    if (rows <= 0 || n <= 0 || groups <= 0 || max_tiles <= 0) return 0;
+    if (form < 0 || form > 2) LLM_FAIL(-1, "gemm_f32_tc: glu form %d is not known", form);
+    if (form == 1 && limit < 0.f) LLM_FAIL(-1, "gemm_f32_tc: the clamp's limit %g is negative", (double)limit);
+    if (llm_gemm_grouped_tile_rows() != kListedRows) LLM_FAIL(-1, "gemm_f32_tc: tiles of %d rows", llm_gemm_grouped_tile_rows());
+    if ((long long)groups * n * 2 > 0x7fffffffLL) LLM_FAIL(-1, "gemm_f32_tc: %d matrices of %d rows are too many", groups, n);
+    Args a{};
+    a.out = out; a.n = n; a.ldc = n; a.swiglu = form ? 1 : 0;
+    a.tiles = tiles; a.clamped = form == 1; a.limit = limit; a.slope = slope; a.row_scale = form == 2 ? row_scale : nullptr;
+    return run(x, source, w, rows, groups, max_tiles, K, planes, a, stream);
 }
 
 LLM_TRACE_EXPORT(gemm_f32_tc)

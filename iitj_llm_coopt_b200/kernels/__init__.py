@@ -82,6 +82,8 @@ _SIGNATURES = {
     "llm_gemm_f32_tc_supported": [_c_int, _c_void_p, _c_void_p],
     "llm_gemm_f32_tc_scratch": [_c_int, _c_int],
     "llm_gemm_f32_tc": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
+    "llm_gemm_f32_tc_listed": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int,
+                               _c_float, _c_float, _c_void_p, _c_void_p, _c_void_p],
     "llm_gemm_bf16_token_tile": [_c_int],
     "llm_gemm_bf16": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p,
                       _c_int, _c_int, _c_int, _c_void_p],
@@ -1170,6 +1172,14 @@ class Kernels:
         form = 0 if not glu else 2 if glu in ("silu", "silu_weighted") else 1
         weighted = glu == "silu_weighted"
         _need(not weighted or plan.get("row_weight") is not None, "moe_linear: the plan holds no row weights")
+        if a.dtype == torch.float32 and self.lib.llm_gemm_f32_tc_supported(k, _ptr(a), _ptr(w)):
+            rows = out.shape[0]
+            planes = torch.empty(self.lib.llm_gemm_f32_tc_scratch(rows, k), dtype=torch.bfloat16, device=a.device)
+            self._call("llm_gemm_f32_tc_listed", _ptr(a), _ptr(plan["source"]) if gather else None, _ptr(w), _ptr(out), rows, n, k,
+                       experts, _ptr(plan["tiles"]), plan["bound"], form, float(limit), float(slope),
+                       _ptr(plan["row_weight"]) if weighted else None, _ptr(planes), self._stream())
+            self.launches += 1
+            return out
         self._call("llm_gemm_grouped", _ptr(a), a.shape[1], 0, 0, _ptr(plan["source"]) if gather else None, _ptr(w), _ptr(out),
                    out.shape[1], 0, 0, DTYPE_CODE[a.dtype], 0, n, k, experts, _ptr(plan["tiles"]), plan["bound"],
                    form, float(limit), float(slope), _ptr(plan["row_weight"]) if weighted else None, None, self._stream())

@@ -96,3 +96,44 @@ def test_on_two_streams_at_once(K):
     for i in range(2):
         for o in outs[i]:
             assert ((o - want[i]).norm() / want[i].norm()).item() < 1e-6
+
+
+# the listed form against the products of each expert by itself (bit for bit) and against 64 bits: tiles of one to 64 rows, experts without
+# rows, choices of experts without tensors, both kernels
+@pytest.mark.parametrize("tokens,experts,top", [(1, 4, 2), (8, 5, 2), (9, 3, 2), (100, 4, 1), (150, 3, 2)])
+@pytest.mark.parametrize("form", [False, "clamped", "silu", "silu_weighted"])
+def test_listed_products(K, tokens, experts, top, form):
+    n, k, pairs = 200, 300, tokens * top
+    g = torch.Generator().manual_seed(tokens)
+    chosen = torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(tokens)]).int()
+    chosen[chosen == 1] = experts                              # nobody at expert 1; those choices have no tensors
+    weights = torch.rand((tokens, top), generator=g).cuda() + 0.5
+    x, w = rnd((tokens, k), 3), rnd((experts, (2 if form else 1) * n, k), 4, k ** -0.5)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    plan = K.moe_plan(chosen.cuda(), experts, torch.zeros(pairs, **i32), torch.empty(pairs, **i32),
+                      torch.empty((K.moe_tile_bound(pairs, experts) + 1, 4), **i32), weights=weights, row_weight=torch.ones(pairs, device="cuda"))
+    out = torch.full((pairs, n), 7.0, device="cuda")
+    K.moe_linear(x, w, out, plan, gather=True, glu=form, limit=1.5, slope=1.7)
+    place = plan["place"].view(tokens, top).cpu()
+    for e in range(experts):
+        at = [(t, j) for t in range(tokens) for j in range(top) if chosen[t, j] == e]
+        if not at:
+            continue
+        rows = torch.tensor([place[t, j] for t, j in at]).cuda()
+        xe = x[torch.tensor([t for t, _ in at]).cuda()].contiguous()
+        y = xe.double() @ w[e].double().t()
+        if form:
+            gate, up = y[:, :n], y[:, n:]
+            if form == "clamped":
+                gate, up = gate.clamp(max=1.5), up.clamp(-1.5, 1.5)
+                y = gate * torch.sigmoid(1.7 * gate) * (up + 1.0)
+            else:
+                s = torch.stack([weights[t, j] for t, j in at]).double().view(-1, 1) if form == "silu_weighted" else 1.0
+                y = torch.nn.functional.silu(s * gate) * (s * up)
+        assert ((out[rows] - y).norm() / y.norm()).item() < 1e-6
+        if form in (False, "silu"):
+            alone = torch.empty(len(at), n, device="cuda")
+            K.linear(xe, w[e], alone, swiglu=bool(form))
+            assert torch.equal(out[rows], alone)
+    live = int((chosen < experts).sum())
+    assert (out[live:] == 7.0).all() and K.gemm_status() == 0
