@@ -222,7 +222,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         uint32_t phase = 1;
         bool free_now = true;                          // what a poll after the box before has found
         for (int b = 0, s = 0; b < boxes; ++b) {
-            if (b >= a.w_stages && !free_now && !mbar_wait(&w_empty[s], phase)) { if (lane == 0) give_up_f32(a, 1); failed = 1; break; }
+            if (b >= a.w_stages && !free_now && !mbar_wait_all(&w_empty[s], phase)) { if (lane == 0) give_up_f32(a, 1); failed = 1; break; }
             if (elect_one()) {
                 unsigned char* st = ring + (size_t)s * kBoxBytes;
                 mbar_expect_tx(&w_full[s], kBoxBytes);
@@ -241,7 +241,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         pdl_wait();
         uint32_t phase = 1;
         for (int j = 0, s = 0; j < n_steps; ++j) {
-            if (j >= a.x_stages && !mbar_wait(&x_empty[s], phase)) { if (lane == 0) give_up_f32(a, 1); failed = 1; break; }
+            if (j >= a.x_stages && !mbar_wait_all(&x_empty[s], phase)) { if (lane == 0) give_up_f32(a, 1); failed = 1; break; }
             if (elect_one()) {
                 mbar_expect_tx(&x_full[s], x_stage);
 #pragma unroll
@@ -263,10 +263,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         for (int i = 0; i < n_steps; ++i) {
             const int c = i / kChunkSteps;
             const bool seg_start = seg_left == a.seg_steps, chunk_start = i % kChunkSteps == 0;
-            bool ok = x_ok || mbar_wait(&x_full[xs], x_phase);
-            if (large && chunk_start && c >= 2) ok = ok && (hi_ok || mbar_wait(&hi_free[c & 1], ((c / 2) - 1) & 1));
-            if (!large && seg_start && i > 0) ok = ok && mbar_wait(&corr_free, (seg++) & 1);
-            ok = ok && (a_ok || mbar_wait(&a_full[as], a_phase));
+            bool ok = x_ok || mbar_wait_all(&x_full[xs], x_phase);
+            if (large && chunk_start && c >= 2) ok = ok && (hi_ok || mbar_wait_all(&hi_free[c & 1], ((c / 2) - 1) & 1));
+            if (!large && seg_start && i > 0) ok = ok && mbar_wait_all(&corr_free, (seg++) & 1);
+            ok = ok && (a_ok || mbar_wait_all(&a_full[as], a_phase));
             if (!ok) { if (lane == 0) give_up_f32(a, 2); failed = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t a0 = t_a + as * kACols, d_hi = t_hi + (c & 1) * a.tt;
@@ -310,7 +310,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         uint32_t phase = 0, a_phase = 1;
         bool w_ok = false;                                     // what a poll during the step before has found
         for (int i = 0, s = group, as = 0; i < n_steps; ++i) {
-            if (!w_ok && !mbar_wait(&w_full[s], phase)) { if (lane == 0) give_up_f32(a, 4); failed = 1; break; }
+            if (!w_ok && !mbar_wait_all(&w_full[s], phase)) { if (lane == 0) give_up_f32(a, 4); failed = 1; break; }
             const unsigned char* st = ring + (size_t)s * kBoxBytes + row * 128;
             // the whole box is taken apart before the wait for the slot, so that only the stores lie between a slot's last product and
             // its next one
@@ -323,19 +323,24 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 split2(v.z, v.w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
             }
             const bool a_ok = __all_sync(0xffffffffu, a_now);
+            __syncwarp();
             if (lane == 0) mbar_arrive(&w_empty[s]);            // the box has been read
+            __syncwarp();
             if ((s += 2) >= a.w_stages) { s -= a.w_stages; phase ^= 1; }
             const bool w_now = mbar_poll(&w_full[s], phase);
-            if (!a_ok && !mbar_wait(&a_empty[as], a_phase)) { if (lane == 0) give_up_f32(a, 4); failed = 1; break; }
+            if (!a_ok && !mbar_wait_all(&a_empty[as], a_phase)) { if (lane == 0) give_up_f32(a, 4); failed = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t ta = t_a + as * kACols + 16 * group + ((uint32_t)(q * 32) << 16);
+            __syncwarp();
             tmem_st16(ta, hi);
             tmem_st16(ta + 32, mid);
             tmem_st16(ta + 64, lo);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             w_ok = __all_sync(0xffffffffu, w_now);
+            __syncwarp();
             if (lane == 0) mbar_arrive(&a_full[as]);
+            __syncwarp();
             if (++as == a.a_slots) { as = 0; a_phase ^= 1; }
         }
     } else if (warp >= kFirstEpi) {
@@ -350,7 +355,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         for (int c = 0; c < n_chunks; ++c) {
             const bool seg_end = --seg_left == 0 || c == n_chunks - 1;
             if (seg_left == 0) seg_left = a.seg_steps / kChunkSteps;
-            if (!mbar_wait(&chunk_full[c & 1], (c / 2) & 1) || (seg_end && !mbar_wait(&corr_full, (seg++) & 1))) { if (lane == 0) give_up_f32(a, 3); failed = 1; ok = false; break; }
+            if (!mbar_wait_all(&chunk_full[c & 1], (c / 2) & 1) || (seg_end && !mbar_wait_all(&corr_full, (seg++) & 1))) { if (lane == 0) give_up_f32(a, 3); failed = 1; ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
             for (int g = 0; g < kCols; g += 8) {
@@ -380,6 +385,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 mbar_arrive(&hi_free[c & 1]);
                 if (seg_end) mbar_arrive(&corr_free);
             }
+            __syncwarp();
         }
         if (a.cluster == 1) {
             pdl_wait();                                    // nothing is stored before the previous kernel has finished

@@ -49,6 +49,25 @@ __device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
         : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return done != 0;
 }
+// The wait of a whole warp: all lanes leave together.  With mbar_wait a phase that ends while its poll is being answered can let some
+// lanes out a poll earlier than others, and the .aligned tensor-memory instructions behind a wait need the warp converged (measured: a
+// few lanes' rows of one step wrong in one of about 10^8 waits).
+__device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity, uint32_t limit = kSpinLimit) {
+    const uint32_t addr = smem_u32(bar);
+    for (uint32_t i = 0; i < limit; ++i) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+        if (__all_sync(0xffffffffu, done)) {
+            __syncwarp();
+            return true;
+        }
+    }
+    return false;
+}
 // True in one lane of the (whole, converged) warp.  A warp that walks its loop together and issues from an elected lane keeps
 // descriptors and addresses in uniform registers; a loop that only one lane walks moves them there for every instruction
 // (measured: 30 clocks an MMA instead of 64).

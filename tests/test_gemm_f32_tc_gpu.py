@@ -137,3 +137,13 @@ def test_listed_products(K, tokens, experts, top, form):
             assert torch.equal(out[rows], alone)
     live = int((chosen < experts).sum())
     assert (out[live:] == 7.0).all() and K.gemm_status() == 0
+
+
+def test_the_same_numbers_every_time(K):
+    """A large product ten times over, bit for bit: 10^8 and more waits of whole warps."""
+    x, w = rnd((2400, 2048), 1), rnd((60000, 2048), 2, 2048 ** -0.5)
+    first, out = torch.empty(2400, 60000, device="cuda"), torch.empty(2400, 60000, device="cuda")
+    K.linear(x, w, first)
+    for _ in range(10):
+        K.linear(x, w, out)
+        assert torch.equal(out, first)
