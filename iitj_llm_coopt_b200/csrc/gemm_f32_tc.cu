@@ -108,6 +108,9 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
     lo = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
 }
 
+// False only if no number behind the pieces `lo` (several pairs' words, or-ed) is infinite or a NaN: those have a NaN there.
+__device__ __forceinline__ bool maybe_not_finite(uint32_t lo) { return (lo & 0x7f80u) == 0x7f80u || (lo & 0x7f800000u) == 0x7f800000u; }
+
 __device__ __forceinline__ float finite_or_zero(float v) { return fabsf(v) <= 3.402823466e38f ? v : 0.f; }
 
 __device__ __forceinline__ float cluster_read(const float* local, uint32_t rank) {
@@ -315,13 +318,19 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             // the whole box is taken apart before the wait for the slot, so that only the stores lie between a slot's last product and
             // its next one
             const bool a_now = i < a.a_slots || mbar_poll(&a_empty[as], a_phase);
-            uint32_t hi[16], mid[16], lo[16];
+            uint32_t hi[16], mid[16], lo[16], all = 0;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const float4 v = *reinterpret_cast<const float4*>(st + ((j ^ sw) << 4));
                 split2(v.x, v.y, hi[2 * j], mid[2 * j], lo[2 * j]);
                 split2(v.z, v.w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
+                all |= lo[2 * j] | lo[2 * j + 1];
             }
+            // The box may be handed back only when its numbers lie in registers: an arrival does not wait for loads that were issued
+            // before it, and beside a kernel that keeps the SM's load path busy they can take longer than the box's successor needs to
+            // land (measured beside attention: rows of a later box in 96 of 96 products of 5 x 2 * 8192 x 2048).  The vote takes a piece
+            // of every number that was read, and the arrival cannot pass what depends on it.
+            if (__any_sync(0xffffffffu, maybe_not_finite(all))) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             const bool a_ok = __all_sync(0xffffffffu, a_now);
             __syncwarp();
             if (lane == 0) mbar_arrive(&w_empty[s]);            // the box has been read

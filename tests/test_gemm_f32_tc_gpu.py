@@ -7,6 +7,8 @@ the rounded sum over at most 160 chunks stay below 1e-6."""
 import pytest
 import torch
 
+import test_attention_f32_gpu
+
 pytestmark = pytest.mark.gpu
 
 
@@ -96,6 +98,33 @@ def test_on_two_streams_at_once(K):
     for i in range(2):
         for o in outs[i]:
             assert ((o - want[i]).norm() / want[i].norm()).item() < 1e-6
+
+
+# beside a kernel that keeps the SMs' load paths or the memory busy: the same bits as alone.  (A box of W that was handed back while its
+# numbers were still on their way into registers was overwritten by its successor here.)
+@pytest.mark.parametrize("other", ["attention", "copies"])
+@pytest.mark.parametrize("tokens", [5, 300])
+def test_beside_other_work(K, tokens, other):
+    q, cache, meta = test_attention_f32_gpu.case(32, 8, 64, 16, [900, 800, 700, 600, 300] * 8, [1] * 40, 5)
+    ctx, a, b = torch.empty(40, 2048, device="cuda"), torch.empty(1 << 27, device="cuda"), torch.empty(1 << 27, device="cuda")
+    x, ws = rnd((tokens, 2048), 1), [rnd((2 * 8192, 2048), 2 + i, 2048 ** -0.5) for i in range(4)]
+    first, outs = [torch.empty(tokens, 8192, device="cuda") for _ in ws], [torch.empty(tokens, 8192, device="cuda") for _ in ws]
+    for w, o in zip(ws, first):
+        K.linear(x, w, o, swiglu=True)
+    assert ((first[0] - product(x, ws[0], True)).norm() / product(x, ws[0], True).norm()).item() < 1e-6
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(25):
+        for w, o in zip(ws, outs):
+            with torch.cuda.stream(side):
+                if other == "copies":
+                    a.copy_(b)
+                else:
+                    for _ in range(8):
+                        K.attention(q, cache, meta, ctx, 32, 8, 64)
+            K.linear(x, w, o, swiglu=True)
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, f) for o, f in zip(outs, first)) and K.gemm_status() == 0
 
 
 # the listed form against the products of each expert by itself (bit for bit) and against 64 bits: tiles of one to 64 rows, experts without
