@@ -6,8 +6,8 @@
 // and the product is the sum of the six piece products that reach 2^-24 of it (hi.hi; hi.mid, mid.hi; mid.mid, hi.lo, lo.hi),
 // accumulated in float32.  The tensor cores cut a sum off where they add to it instead of rounding it, which would cost
 // precision along a long k range; therefore the large piece product (hi.hi) stays in tensor memory for 128 k at a time (eight
-// instructions), and these chunks are added in registers, rounded to nearest.  The five small products (2^-8 of the sum) have
-// accumulators of their own for a whole segment of the k range.  Relative error (2-norm, against 64 bits, normal factors) at
+// instructions), and these chunks are added in registers, rounded to nearest.  The five small products (2^-8 of the sum; lo.mid
+// rides along) have accumulators of their own for a whole segment of the k range.  Relative error (2-norm, against 64 bits, normal factors) at
 // K = 128 / 512 / 2048 / 8192: 1.2e-7 / 1.3e-7 / 1.5e-7 / 1.9e-7; a chain of fused multiply-adds has 2.0e-7 / 4.0e-7 / 8.0e-7 / 1.6e-6.
 //
 // Order of a sum: chunks of 128 k in order, the small products of a segment with the last chunk of the segment.  Segments
@@ -282,15 +282,17 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     umma_commit(&x_empty[xs]);
                     if (i % kChunkSteps == kChunkSteps - 1 || last) umma_commit(&chunk_full[c & 1]);
                 } else {
-                    // the pieces of x lie one after the other, so that one instruction multiplies a piece of W with two of them:
-                    // the small products of order 2^-8 add up in one half of t_corr, those of order 2^-16 in the other
+                    // The pieces of x lie one after the other, so that one instruction multiplies a piece of W with two of them and adds to
+                    // both halves of t_corr.  All three have one shape and one accumulator: only such instructions are promised to run in
+                    // the order of their issue (lo.hi by itself, half as wide, was not).  Five instructions of one product each cost a
+                    // step of five tokens 2.23 ms against 2.22; lo.mid comes with the width and is below what the sum can hold.
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         const uint32_t ah = a0 + 8 * k, am = ah + 32, al = ah + 64;
                         const uint64_t bh = desc + 2 * k, bm = bh + plane;
                         umma_ts(t_corr, ah, bm, idesc2, !(seg_start && k == 0));          // hi.mid | hi.lo
                         umma_ts(t_corr, am, bh, idesc2, 1u);                              // mid.hi | mid.mid
-                        umma_ts(t_corr + a.tt, al, bh, idesc1, 1u);                       //        | lo.hi
+                        umma_ts(t_corr, al, bh, idesc2, 1u);                              // lo.hi  | lo.mid
                     }
                     umma_commit(&a_empty[as]);
                     umma_commit(&x_empty[xs]);

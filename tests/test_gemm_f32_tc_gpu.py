@@ -100,6 +100,22 @@ def test_on_two_streams_at_once(K):
             assert ((o - want[i]).norm() / want[i].norm()).item() < 1e-6
 
 
+# sums whose large pieces cancel: what is left are the small products, and not one of them is missing.  All pieces' sums of these factors are
+# held exactly, and 24 roundings of numbers below one (chunks and segments) are off by 24 * 2^-25 = 7e-7; sixteen low pieces, as one
+# instruction adds them, are worth 1e-5.
+@pytest.mark.parametrize("tokens", [5, 60, 100])
+def test_small_products_are_all_there(K, tokens):
+    k, n = 2048, 300
+    sign = torch.ones(k, device="cuda")
+    sign[1::2] = -1.0
+    rest = lambda rows, seed: torch.randint(-2 ** 14, 2 ** 14, (rows, k), generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda") * 2.0 ** -23
+    for x, w in ((torch.ones(tokens, k, device="cuda"), sign * (1.0 + rest(n, 1))), (sign * (1.0 + rest(tokens, 2)), torch.ones(n, k, device="cuda"))):
+        x, w, out = x.contiguous(), w.contiguous(), torch.empty(tokens, n, device="cuda")
+        for _ in range(20):
+            K.linear(x, w, out)
+            assert (out - product(x, w)).abs().max().item() < 1e-6
+
+
 # beside a kernel that keeps the SMs' load paths or the memory busy: the same bits as alone.  (A box of W that was handed back while its
 # numbers were still on their way into registers was overwritten by its successor here.)
 @pytest.mark.parametrize("other", ["attention", "copies"])
