@@ -35,8 +35,8 @@
 // Listed form (llm_gemm_f32_tc_listed): the rows were sorted by weight matrix on the device (the experts of a routed feed-forward);
 // a block takes its tile from the list, blocks beyond the list's count leave at once.
 //
-// Infinities and NaNs arrive through hi.hi as they would in a plain product; the small products, which then hold inf - inf, are left
-// out when they are not finite.  Waits are bounded: a wait that runs out records a code in the status word of the bfloat16 product
+// Infinities and NaNs arrive through hi.hi as they would in a plain product (a NaN gets its quiet bit in hi first); the small products,
+// which then hold inf - inf, are left out when they are not finite.  Waits are bounded: a wait that runs out records a code in the status word of the bfloat16 product
 // (1 producer, 2 issuer, 3 epilogue, 4 converter), and the block falls through to its teardown.
 #include "tcgen05_common.cuh"
 
@@ -110,6 +110,11 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
 
 // False only if no number behind the pieces `lo` (several pairs' words, or-ed) is infinite or a NaN: those have a NaN there.
 __device__ __forceinline__ bool maybe_not_finite(uint32_t lo) { return (lo & 0x7f80u) == 0x7f80u || (lo & 0x7f800000u) == 0x7f800000u; }
+// The quiet bits of those of two numbers that are NaNs, where hi has them: a NaN whose payload lies in the 16 bits that are cut off
+// would become an infinity.
+__device__ __forceinline__ uint32_t quiet_nan2(uint32_t a, uint32_t b) {
+    return ((a & 0x7fffffffu) > 0x7f800000u ? 0x40u : 0u) | ((b & 0x7fffffffu) > 0x7f800000u ? 0x400000u : 0u);
+}
 
 __device__ __forceinline__ float finite_or_zero(float v) { return fabsf(v) <= 3.402823466e38f ? v : 0.f; }
 
@@ -332,7 +337,16 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             // before it, and beside a kernel that keeps the SM's load path busy they can take longer than the box's successor needs to
             // land (measured beside attention: rows of a later box in 96 of 96 products of 5 x 2 * 8192 x 2048).  The vote takes a piece
             // of every number that was read, and the arrival cannot pass what depends on it.
-            if (__any_sync(0xffffffffu, maybe_not_finite(all))) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            if (__any_sync(0xffffffffu, maybe_not_finite(all))) {
+#pragma unroll 1
+                for (int j = 0; j < 8; ++j) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(st + ((j ^ sw) << 4));
+                    const uint32_t first = quiet_nan2(v.x, v.y), second = quiet_nan2(v.z, v.w);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) hi[i] |= i == 2 * j ? first : i == 2 * j + 1 ? second : 0u;
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // (these loads, too, come before the box's successor)
+            }
             const bool a_ok = __all_sync(0xffffffffu, a_now);
             __syncwarp();
             if (lane == 0) mbar_arrive(&w_empty[s]);            // the box has been read
@@ -471,6 +485,8 @@ split_planes_kernel(const float* __restrict__ x, bf16* __restrict__ planes, int 
         uint2 h, m, l;
         split2(v.x, v.y, h.x, m.x, l.x);
         split2(v.z, v.w, h.y, m.y, l.y);
+        h.x |= quiet_nan2(__float_as_uint(v.x), __float_as_uint(v.y));
+        h.y |= quiet_nan2(__float_as_uint(v.z), __float_as_uint(v.w));
         bf16* d = planes + (size_t)t * kp + k;
         *reinterpret_cast<uint2*>(d) = h;
         *reinterpret_cast<uint2*>(d + plane) = m;

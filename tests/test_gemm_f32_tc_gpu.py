@@ -74,6 +74,23 @@ def test_infinities_and_nans_go_where_they_would(K):
         assert ((out - want[rows])[ok].abs() <= 1e-5 * want[rows][ok].abs() + 1e-4).all()
 
 
+@pytest.mark.parametrize("tokens", [8, 40])
+def test_nans_stay_nans_whatever_their_payload(K, tokens):
+    x, w = rnd((tokens, 300), 3), rnd((70, 300), 4)
+    bits = torch.tensor([0x7f800001, 0x7fc00000, -0x7fffff, 0x7f80ffff, -1], dtype=torch.int64).int().cuda()     # low, high, negative, all low bits
+    for i, at in enumerate((0, 33, 131, 255, 299)):
+        x.view(torch.int32)[i, at] = bits[i]
+        w.view(torch.int32)[7 * i, at] = bits[4 - i]
+    w[69, 100], x[6, 7] = float("inf"), float("inf")             # infinities beside them stay infinite
+    want = (x.double() @ w.double().t()).float()
+    out = torch.empty(tokens, 70, device="cuda")
+    K.linear(x, w, out)
+    assert want.isnan().any() and want.isinf().any()
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isposinf(), want.isposinf()) and torch.equal(out.isneginf(), want.isneginf())
+    ok = want.isfinite()
+    assert ((out - want)[ok].abs() <= 1e-5 * want[ok].abs() + 1e-4).all()
+
+
 def test_rows_that_start_off_a_boundary_take_the_other_kernel(K):
     base = rnd((5 * 64 + 1,), 5)
     x, w = base[1:].view(5, 64), rnd((30, 64), 6)
