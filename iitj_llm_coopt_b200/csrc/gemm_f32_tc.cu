@@ -9,8 +9,11 @@
 // instructions), and these chunks are added in registers, rounded to nearest.  The five small products (2^-8 of the sum; lo.mid
 // rides along) have accumulators of their own for a whole segment of the k range.  Relative error (2-norm, against 64 bits, normal factors) at
 // K = 128 / 512 / 2048 / 8192: 1.2e-7 / 1.3e-7 / 1.5e-7 / 1.9e-7; a chain of fused multiply-adds has 2.0e-7 / 4.0e-7 / 8.0e-7 / 1.6e-6.
+// Factors of one sign, whose sums shrink with every cut: K = 64 / 256 / 2048 0.9e-7 / 1.8e-7 / 1.8e-7 against 1.2e-7 / 2.5e-7 / 6.9e-7;
+// a first chunk of 128 k was as far off as the chain up to K = 132 (1.81e-7 against 1.75e-7 at 128), so K up to 192 has chunks of 64.
+// Numbers below 2^-110 lose bits: the last of their pieces lie below the smallest bfloat16 number, 2^-133.
 //
-// Order of a sum: chunks of 128 k in order, the small products of a segment with the last chunk of the segment.  Segments
+// Order of a sum: chunks of 128 k (64 up to K = 192) in order, the small products of a segment with the last chunk of the segment.  Segments
 // depend on K alone (an eighth of it, at least 256), so an output element is the same whatever else is in the call and
 // however the call is cut into tiles and blocks.
 //
@@ -49,7 +52,8 @@ typedef __nv_bfloat16 bf16;
 constexpr int kRows = 128;               // rows of W per block (UMMA M)
 constexpr int kStepK = 64;               // k of a step: two boxes of W of 32 float32 a row
 constexpr int kBoxBytes = kRows * 32 * 4;
-constexpr int kChunkSteps = 2;           // steps whose hi.hi products stay in one accumulator
+constexpr int kChunkSteps = 2;           // steps whose hi.hi products stay in one accumulator ...
+constexpr int kShortSteps = 3;           // ... but one where the k range has at most so many
 // Ring stages; of W: boxes, an even number, so that a stage is always read by the same group of converters.  (Boxes land in any
 // order: a group that shared a stage could come to wait for the stage's second box before the first, the other group's, had landed,
 // and a wait by parity that is two phases early passes at once.)
@@ -167,8 +171,8 @@ __device__ __forceinline__ float glu(const Args& a, float g, float u, int r) {
 }
 
 // SMALL: one tile of at most 16 tokens; fewer threads of fewer registers, so that two blocks share an SM and the next product's
-// blocks can start on their weights while this one's finish.
-template <bool SMALL>
+// blocks can start on their weights while this one's finish.  CHUNK: steps of a chunk.
+template <bool SMALL, int CHUNK>
 __global__ void __launch_bounds__(SMALL ? 512 : 640, SMALL ? 2 : 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Args a) {
     constexpr int kEpiWarps = SMALL ? 4 : 8;
@@ -200,7 +204,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
     const int block_steps = a.segs / a.cluster * a.seg_steps;
     const int step0 = rank * block_steps, n_steps = min(a.steps - step0, block_steps);
-    const int n_chunks = (n_steps + kChunkSteps - 1) / kChunkSteps;
+    const int n_chunks = (n_steps + CHUNK - 1) / CHUNK;
     const int x_stage = 3 * a.tt * 128;                // a stage of x: 64 k of the three pieces
 
     if (threadIdx.x == 0) {
@@ -269,8 +273,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         int xs = 0, as = 0, seg_left = a.seg_steps, seg = 0;
         bool x_ok = false, a_ok = false, hi_ok = false;       // what a poll during the step before has found
         for (int i = 0; i < n_steps; ++i) {
-            const int c = i / kChunkSteps;
-            const bool seg_start = seg_left == a.seg_steps, chunk_start = i % kChunkSteps == 0;
+            const int c = i / CHUNK;
+            const bool seg_start = seg_left == a.seg_steps, chunk_start = i % CHUNK == 0;
             bool ok = x_ok || mbar_wait_all(&x_full[xs], x_phase);
             if (large && chunk_start && c >= 2) ok = ok && (hi_ok || mbar_wait_all(&hi_free[c & 1], ((c / 2) - 1) & 1));
             if (!large && seg_start && i > 0) ok = ok && mbar_wait_all(&corr_free, (seg++) & 1);
@@ -285,7 +289,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     for (int k = 0; k < 4; ++k) umma_ts(d_hi, a0 + 8 * k, desc + 2 * k, idesc1, !(chunk_start && k == 0));
                     umma_commit(&a_empty[as]);
                     umma_commit(&x_empty[xs]);
-                    if (i % kChunkSteps == kChunkSteps - 1 || last) umma_commit(&chunk_full[c & 1]);
+                    if (i % CHUNK == CHUNK - 1 || last) umma_commit(&chunk_full[c & 1]);
                 } else {
                     // The pieces of x lie one after the other, so that one instruction multiplies a piece of W with two of them and adds to
                     // both halves of t_corr.  All three have one shape and one accumulator: only such instructions are promised to run in
@@ -309,7 +313,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             if (++xs == a.x_stages) { xs = 0; x_phase ^= 1; desc = desc0; }
             if (++as == a.a_slots) { as = 0; a_phase ^= 1; }
             if (--seg_left == 0) seg_left = a.seg_steps;
-            const int cn = (i + 1) / kChunkSteps;
+            const int cn = (i + 1) / CHUNK;
             const bool x_now = mbar_poll(&x_full[xs], x_phase), a_now = mbar_poll(&a_full[as], a_phase);
             const bool hi_now = large && cn >= 2 && mbar_poll(&hi_free[cn & 1], ((cn / 2) - 1) & 1);
             x_ok = __all_sync(0xffffffffu, x_now); a_ok = __all_sync(0xffffffffu, a_now); hi_ok = __all_sync(0xffffffffu, hi_now);
@@ -376,10 +380,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
         for (int j = 0; j < kCols; ++j) total[j] = 0.f;
         bool ok = true;
-        int seg_left = a.seg_steps / kChunkSteps, seg = 0;
+        int seg_left = a.seg_steps / CHUNK, seg = 0;
         for (int c = 0; c < n_chunks; ++c) {
             const bool seg_end = --seg_left == 0 || c == n_chunks - 1;
-            if (seg_left == 0) seg_left = a.seg_steps / kChunkSteps;
+            if (seg_left == 0) seg_left = a.seg_steps / CHUNK;
             if (!mbar_wait_all(&chunk_full[c & 1], (c / 2) & 1) || (seg_end && !mbar_wait_all(&corr_full, (seg++) & 1))) { if (lane == 0) give_up_f32(a, 3); failed = 1; ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
@@ -448,8 +452,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         llm_cluster_sync();                                // every block's chunk sums lie in its shared memory
         pdl_wait();
         const int rows = a.swiglu ? kRows / 2 : kRows, live = tok_end - tok0;
-        const int all_chunks = (a.steps + kChunkSteps - 1) / kChunkSteps;
-        const int per_block = a.segs / a.cluster * (a.seg_steps / kChunkSteps);         // (the last block may have fewer)
+        const int all_chunks = (a.steps + CHUNK - 1) / CHUNK;
+        const int per_block = a.segs / a.cluster * (a.seg_steps / CHUNK);         // (the last block may have fewer)
         const int l = (threadIdx.x >> 3) & 3, per_pass = blockDim.x / 4, stride = a.tt * kRows;
         for (int e0 = rank * per_pass; e0 < live * rows; e0 += a.cluster * per_pass) {
             const int e = e0 + (threadIdx.x >> 5) * 8 + (threadIdx.x & 7);
@@ -541,9 +545,9 @@ Plan make_plan(int tokens, int n, int swiglu, int steps, int seg_steps, int sms,
     return best;
 }
 
-template <bool SMALL>
+template <bool SMALL, int CHUNK>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& a, dim3 grid, int smem, cudaStream_t stream) {
-    auto kern = gemm_f32_tc_kernel<SMALL>;
+    auto kern = gemm_f32_tc_kernel<SMALL, CHUNK>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
     if (e != cudaSuccess) LLM_FAIL(-2, "gemm_f32_tc: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     if (a.cluster > 1)
@@ -599,7 +603,9 @@ int run(const float* x, const int* source, const float* w, int tokens, int group
     const int blocks = (int)((quads + 255) / 256 < 148 * 8 ? (quads + 255) / 256 : 148 * 8);
     llm_launch(split_planes_kernel, blocks, 256, 0, stream, x, (bf16*)planes, tokens, K, kp, source, a.tiles ? a.tiles + 1 : nullptr);
     LLM_CHECK_LAUNCH("gemm_f32_tc_planes");
-    return tile_tokens <= kSmallTokens ? launch<true>(mw, mx, a, grid, p.smem, stream) : launch<false>(mw, mx, a, grid, p.smem, stream);
+    const auto go = a.steps <= kShortSteps ? (tile_tokens <= kSmallTokens ? launch<true, 1> : launch<false, 1>)
+                                           : (tile_tokens <= kSmallTokens ? launch<true, kChunkSteps> : launch<false, kChunkSteps>);
+    return go(mw, mx, a, grid, p.smem, stream);
 }
 
 }  // namespace

@@ -117,6 +117,20 @@ def test_on_two_streams_at_once(K):
             assert ((o - want[i]).norm() / want[i].norm()).item() < 1e-6
 
 
+# against 64 bits no further off than the chain of fused multiply-adds that takes the other rows, for random signs and (the tensor cores cut
+# sums off instead of rounding them) for factors of one sign; from K = 256 on the chain loses more with every number
+@pytest.mark.parametrize("k", [4, 8, 16, 32, 48, 64, 68, 96, 128, 132, 160, 192, 256, 2048])
+@pytest.mark.parametrize("one_sign", [False, True])
+def test_no_further_off_than_a_chain(K, k, one_sign):
+    x, w = rnd((96, k), 1), rnd((512, k), 2)
+    if one_sign:
+        x, w = x.abs(), w.abs()
+    want, out, chain = product(x, w), torch.empty(96, 512, device="cuda"), torch.empty(96, 512, device="cuda")
+    K.linear(x, w, out)
+    K._call("llm_gemm_f32", x.data_ptr(), w.data_ptr(), chain.data_ptr(), 96, 512, k, k, k, 512, 0, K._stream())
+    assert (out - want).norm().item() <= (chain - want).norm().item()
+
+
 # sums whose large pieces cancel: what is left are the small products, and not one of them is missing.  All pieces' sums of these factors are
 # held exactly, and 24 roundings of numbers below one (chunks and segments) are off by 24 * 2^-25 = 7e-7; sixteen low pieces, as one
 # instruction adds them, are worth 1e-5.
