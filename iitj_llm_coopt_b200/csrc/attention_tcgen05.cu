@@ -544,9 +544,11 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
 // Adds the partial results of a query tile's key splits: out = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M).
 // D / 4 lanes per (query row, head), four output dims a lane and all loads asked for at once; splits that got no key tile are left out
-// by index; a tile that was not split needs nothing.  Bound by the latency of its loads: with a block per row and head and a number a
-// thread, 512 rows x 24 heads of 128 dims in four splits (25 MB) took 27.8 us in 12288 blocks.
-// MAX bounds the splits (4, 8 or 16): a thread holds as many rows of partial results, and fewer of them let more threads share an SM.
+// by index; a tile that was not split needs nothing.  Bound by the latency of its loads.  Measured back to back, against a block per
+// row and head and a number a thread: 512 rows x 24 heads of 128 dims in 4 splits (25 MB) 22.2 -> 4.8 us, 256 rows in 8 splits
+// 12.8 -> 5.2, 128 rows in 16 splits 8.1 -> 7.0; 32 heads of 64 dims, 512 rows in 4 splits 18.4 -> 3.6, 128 rows in 16 splits 6.6 -> 4.6.
+// MAX bounds the splits (4, 8 or 16): a thread holds as many rows of partial results, and fewer of them let more threads share an SM
+// (38, 64 and 128 registers; at 16 one of them is spilled, and two blocks share an SM).
 constexpr int kMaxKeySplits = 16;
 constexpr int kMergeThreads = 256;
 
