@@ -38,15 +38,19 @@ class RequestOutput:
 
 def workspace_bytes_estimate(spec, tokens: int, rows: int, itemsize: int) -> int:
     """Rough size of the step's scratch tensors for `tokens` tokens and `rows` logits rows (twice what the
-    shapes need: the workspace grows its buffers to powers of two)."""
-    widest = 0
+    shapes need: the workspace grows its buffers to powers of two).  In float32 with the bfloat16 pieces of the
+    longest row of a product, 6 bytes a number (csrc/gemm_f32_tc.cu; with routed experts a row per choice)."""
+    widest = longest = 0
     for layer in spec.layers:
         cols = 3 * spec.width
         for _name, ps in layer.parts:        # whatever sizes the layer's parts name: projections, inner widths
             heads, kv_heads, head_dim = (getattr(ps, a, 0) or 0 for a in ("heads", "kv_heads", "head_dim"))
             cols += (2 * heads + 2 * kv_heads) * head_dim + 3 * (getattr(ps, "inner", 0) or 0)
+            top = getattr(ps, "experts_per_token", 0) or 1
+            longest = max(longest, heads * max(head_dim, getattr(ps, "value_dim", 0) or 0), top * max(spec.width, getattr(ps, "inner", 0) or 0))
         widest = max(widest, cols)
-    return 2 * (tokens * (widest * itemsize + 4 * spec.width) + rows * spec.vocab * 4) + (64 << 20)
+    pieces = 6 * longest if itemsize == 4 else 0
+    return 2 * (tokens * (widest * itemsize + 4 * spec.width + pieces) + rows * spec.vocab * 4) + (64 << 20)
 
 
 def build_engine(model: str | None = None, engine_config: EngineConfig | None = None, *, config=None,

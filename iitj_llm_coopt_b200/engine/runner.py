@@ -62,6 +62,8 @@ class ModelRunner:
         self._meta = None            # int32 device buffer the step's index arrays live in
         self._copied = None          # event: the last host-to-device copy of the staging buffer is done
         self._capture_stream = None  # side stream that graph captures are recorded on
+        self._graph_pool = None      # memory that the captured graphs share: what a step allocates and gives back (pieces of
+        #                              float32 rows) is there once, not once per graph; graphs are replayed one after the other
         self.steps = 0
         self.copied_bytes = 0
         self._preparer_list = None
@@ -116,6 +118,8 @@ class ModelRunner:
         generation = self._generation()
         self.graph_captures += 1
         graph = torch.cuda.CUDAGraph()
+        if not self._graphs:                     # (a pool lives as long as a graph holds it)
+            self._graph_pool = torch.cuda.graph_pool_handle()
         # The garbage collector must not run inside the capture: collecting an older engine there would
         # destroy its graphs, which CUDA forbids while a capture is open and which voids the capture.
         # The capture is opened by hand rather than with torch.cuda.graph(), which first waits for the whole
@@ -127,7 +131,7 @@ class ModelRunner:
         self._capture_stream.wait_stream(torch.cuda.current_stream())
         try:
             with torch.cuda.stream(self._capture_stream):
-                graph.capture_begin(capture_error_mode="thread_local")
+                graph.capture_begin(pool=self._graph_pool, capture_error_mode="thread_local")
                 try:
                     logits = self.model.forward(ctx)
                 finally:
