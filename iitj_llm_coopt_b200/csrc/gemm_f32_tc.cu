@@ -40,7 +40,7 @@
 //
 // Infinities and NaNs arrive through hi.hi as they would in a plain product (a NaN gets its quiet bit in hi first); the small products,
 // which then hold inf - inf, are left out when they are not finite.  Waits are bounded: a wait that runs out records a code in the status word of the bfloat16 product
-// (1 producer, 2 issuer, 3 epilogue, 4 converter), and the block falls through to its teardown.
+// (11 producer, 12 issuer, 13 epilogue, 14 converter), and the block falls through to its teardown.
 #include "tcgen05_common.cuh"
 
 LLM_API int llm_gemm_grouped_tile_rows();      // gemm_grouped.cu
@@ -234,7 +234,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         uint32_t phase = 1;
         bool free_now = true;                          // what a poll after the box before has found
         for (int b = 0, s = 0; b < boxes; ++b) {
-            if (b >= a.w_stages && !free_now && !mbar_wait_all(&w_empty[s], phase)) { if (lane == 0) give_up_f32(a, 1); failed = 1; break; }
+            if (b >= a.w_stages && !free_now && !mbar_wait_all(&w_empty[s], phase)) { if (lane == 0) give_up_f32(a, 11); failed = 1; break; }
             if (elect_one()) {
                 unsigned char* st = ring + (size_t)s * kBoxBytes;
                 mbar_expect_tx(&w_full[s], kBoxBytes);
@@ -253,7 +253,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         pdl_wait();
         uint32_t phase = 1;
         for (int j = 0, s = 0; j < n_steps; ++j) {
-            if (j >= a.x_stages && !mbar_wait_all(&x_empty[s], phase)) { if (lane == 0) give_up_f32(a, 1); failed = 1; break; }
+            if (j >= a.x_stages && !mbar_wait_all(&x_empty[s], phase)) { if (lane == 0) give_up_f32(a, 11); failed = 1; break; }
             if (elect_one()) {
                 mbar_expect_tx(&x_full[s], x_stage);
 #pragma unroll
@@ -279,7 +279,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             if (large && chunk_start && c >= 2) ok = ok && (hi_ok || mbar_wait_all(&hi_free[c & 1], ((c / 2) - 1) & 1));
             if (!large && seg_start && i > 0) ok = ok && mbar_wait_all(&corr_free, (seg++) & 1);
             ok = ok && (a_ok || mbar_wait_all(&a_full[as], a_phase));
-            if (!ok) { if (lane == 0) give_up_f32(a, 2); failed = 1; break; }
+            if (!ok) { if (lane == 0) give_up_f32(a, 12); failed = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t a0 = t_a + as * kACols, d_hi = t_hi + (c & 1) * a.tt;
             const bool last = i == n_steps - 1;
@@ -324,7 +324,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         uint32_t phase = 0, a_phase = 1;
         bool w_ok = false;                                     // what a poll during the step before has found
         for (int i = 0, s = group, as = 0; i < n_steps; ++i) {
-            if (!w_ok && !mbar_wait_all(&w_full[s], phase)) { if (lane == 0) give_up_f32(a, 4); failed = 1; break; }
+            if (!w_ok && !mbar_wait_all(&w_full[s], phase)) { if (lane == 0) give_up_f32(a, 14); failed = 1; break; }
             const unsigned char* st = ring + (size_t)s * kBoxBytes + row * 128;
             // the whole box is taken apart before the wait for the slot, so that only the stores lie between a slot's last product and
             // its next one
@@ -357,7 +357,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             __syncwarp();
             if ((s += 2) >= a.w_stages) { s -= a.w_stages; phase ^= 1; }
             const bool w_now = mbar_poll(&w_full[s], phase);
-            if (!a_ok && !mbar_wait_all(&a_empty[as], a_phase)) { if (lane == 0) give_up_f32(a, 4); failed = 1; break; }
+            if (!a_ok && !mbar_wait_all(&a_empty[as], a_phase)) { if (lane == 0) give_up_f32(a, 14); failed = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t ta = t_a + as * kACols + 16 * group + ((uint32_t)(q * 32) << 16);
             __syncwarp();
@@ -384,7 +384,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         for (int c = 0; c < n_chunks; ++c) {
             const bool seg_end = --seg_left == 0 || c == n_chunks - 1;
             if (seg_left == 0) seg_left = a.seg_steps / CHUNK;
-            if (!mbar_wait_all(&chunk_full[c & 1], (c / 2) & 1) || (seg_end && !mbar_wait_all(&corr_full, (seg++) & 1))) { if (lane == 0) give_up_f32(a, 3); failed = 1; ok = false; break; }
+            if (!mbar_wait_all(&chunk_full[c & 1], (c / 2) & 1) || (seg_end && !mbar_wait_all(&corr_full, (seg++) & 1))) { if (lane == 0) give_up_f32(a, 13); failed = 1; ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
             for (int g = 0; g < kCols; g += 8) {

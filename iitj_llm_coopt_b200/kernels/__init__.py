@@ -200,7 +200,8 @@ _SIGNATURES = {
 
 # The library's health words in the order llm_sample copies them out (csrc/common.cuh): which kernel, and what its codes mean.
 HEALTH_WORDS = (
-    ("tcgen05 matrix product", "a bounded wait ran out (1 producer, 2 MMA issuer, 3 epilogue)"),
+    ("tcgen05 matrix product", "a bounded wait ran out (bfloat16: 1 producer, 2 MMA issuer, 3 epilogue; float32: 11 producer, 12 MMA issuer, "
+                               "13 epilogue, 14 taking the weights apart)"),
     ("CTA-pair matrix product", "a bounded wait ran out (1 producer, 2 MMA issuer, 3 epilogue, 4 drained accumulator, "
                                 "5 other clusters' partial sums)"),
     ("tcgen05 prefill attention", "a bounded wait ran out (1 to 8), or a key's score lay more than 2^100 above all keys of "

@@ -23,3 +23,14 @@ def test_a_failed_kernel_stops_the_engine(model_dirs):
     s2 = other.new_sequence([5, 6, 7, 8], 3, 0.0, True)
     other.run_until_done()
     assert s2.finished and len(s2.tokens) == 7
+
+
+@pytest.mark.parametrize("codes,words", [((14 << 16 | 3, 0, 0, 0), ("matrix product", "code 14 in block/item 3", "14 taking the weights apart")),
+                                         ((0, 0, 0, 7 << 16 | 9), ("decode attention", "code 7 in block/item 9"))])
+def test_the_message_names_the_kernel_and_the_wait(codes, words):
+    from types import SimpleNamespace
+    from iitj_llm_coopt_b200.kernels import KernelError, Kernels
+    fake = SimpleNamespace(gemm_status=lambda: 0, gemm_pair_status=lambda: 0, attention_status=lambda: 0, decode_status=lambda: 0, _pair_counters={})
+    with pytest.raises(KernelError) as failure:
+        Kernels.check_health(fake, codes)
+    assert all(w in str(failure.value) for w in words)
