@@ -206,7 +206,6 @@ LLM_API int llm_token_shift(const void* x, const float* mu, const float* before,
 LLM_API int llm_wkv_decay(const float* low, const float* w2, const float* w0, float* out, int tokens, int channels, int rank,
                           cudaStream_t stream) {
     if (tokens == 0) return 0;
-    if ((size_t)rank * sizeof(float) > 48 * 1024) LLM_FAIL(-1, "wkv_decay: rank %d is too large", rank);
     const int c_blocks = (channels + kDecayThreads - 1) / kDecayThreads;
     if (c_blocks > 65535) LLM_FAIL(-1, "wkv_decay: %d channels are too many for one launch", channels);
     llm_launch(wkv_decay_kernel, dim3((unsigned)((tokens + kDecayTokens - 1) / kDecayTokens), c_blocks), kDecayThreads, 0, stream, low, w2, w0, out,

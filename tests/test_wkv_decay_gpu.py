@@ -20,3 +20,16 @@ def test_decay(tokens, channels, rank):
     K.wkv_decay(low, w2, w0, out[:tokens])
     want = torch.exp(-torch.exp(torch.tanh(low.double()) @ w2.double().t() + w0.double()))
     assert (out[:tokens] - want).abs().max().item() < 1e-5 and (out[tokens] == 7.0).all()
+
+
+def test_a_rank_that_one_block_could_not_hold():
+    """12300 numbers a channel.  A running sum of about one is rounded 12300 times by at most 2^-24 of itself, up or down at random: about
+    111 * 6e-8 = 7e-6, and 5e-5 is beyond the luck of 2210 sums; through both exponentials it grows by less than one."""
+    from iitj_llm_coopt_b200 import kernels
+    K = kernels.load()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    low, w2 = torch.randn((17, 12300), generator=g, device="cuda"), torch.randn((130, 12300), generator=g, device="cuda") * 0.01
+    w0, out = torch.randn(130, generator=g, device="cuda") - 1.0, torch.empty(17, 130, device="cuda")
+    K.wkv_decay(low, w2, w0, out)
+    want = torch.exp(-torch.exp(torch.tanh(low.double()) @ w2.double().t() + w0.double()))
+    assert (out - want).abs().max().item() < 5e-5
