@@ -49,9 +49,9 @@ __device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
         : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return done != 0;
 }
-// The wait of a whole warp: all lanes leave together.  With mbar_wait a phase that ends while its poll is being answered can let some
-// lanes out a poll earlier than others, and the .aligned tensor-memory instructions behind a wait need the warp converged (measured: a
-// few lanes' rows of one step wrong in one of about 10^8 waits).
+// The wait of a whole warp: its lanes leave together, converged for the .aligned tensor-memory instructions behind it.  (With mbar_wait
+// lanes may leave in different polls and meet again where the compiler joins them.  No wrong result has been traced to that: the
+// bfloat16 kernels wait that way, and their results beside attention and copies on other streams are the same bits as alone.)
 __device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity, uint32_t limit = kSpinLimit) {
     const uint32_t addr = smem_u32(bar);
     for (uint32_t i = 0; i < limit; ++i) {
