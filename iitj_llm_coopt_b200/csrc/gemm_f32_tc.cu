@@ -30,10 +30,11 @@
 // Products with few tiles share the k range out over a cluster of blocks (segments whole): every block keeps the sums of its
 // chunks in shared memory, and the blocks then add all chunks of their part of the tile in order, over distributed shared memory.
 //
-// What bounds it: a decode step the HBM bytes of W, a prompt the tensor cores at six bfloat16 products per float32 product (278
-// TFLOP/s of the measured bf16 rate) and the barriers above.  Measured, cold weights, against the product on the CUDA cores
-// (gemm_f32.cu): 5 tokens, 2048 x 2048 195 -> 9 us, 2048 x 8192 770 -> 36 us, 128256 x 2048 1006 -> 173 us (6.1 TB/s);
-// 777 tokens, 2048 x 2048 256 -> 66 us, 2048 x 8192 993 -> 196 us (133 TFLOP/s), SwiGLU 8192 x 2048 1483 -> 331 us (157 TFLOP/s).
+// What bounds it: a decode step the HBM bytes of W, a prompt the tensor cores at seven bfloat16 products per float32 product (six of
+// them of use: 278 TFLOP/s of the measured bf16 rate) and the barriers above.  Measured with the planes, cold weights, against the
+// product on the CUDA cores (gemm_f32.cu): 5 tokens, 2048 x 2048 195 -> 10 us, 2048 x 8192 770 -> 34 us; one token, 128256 x 2048
+// 1006 -> 172 us (6.1 TB/s); 777 tokens, 2048 x 2048 256 -> 69 us, 2048 x 8192 993 -> 214 us (122 TFLOP/s), SwiGLU 8192 x 2048 1483 ->
+// 356 us (146 TFLOP/s; 331 us before boxes were handed back after the vote and the small products had one shape).
 //
 // Listed form (llm_gemm_f32_tc_listed): the rows were sorted by weight matrix on the device (the experts of a routed feed-forward);
 // a block takes its tile from the list, blocks beyond the list's count leave at once.
