@@ -231,6 +231,209 @@ __global__ void talking_attn_kernel(const T* __restrict__ q, int q_stride, const
     }
 }
 
+// ---- few tokens: a cluster of blocks a token -----------------------------------------------------------------------
+// The kernel above works on a decoded token with one block, whose 16 warps walk 32 heads and all their keys and values by
+// themselves (a lone token of 32 heads of 128 numbers: 41 us, of which the loads are 256 KiB through one SM).  Here the heads are shared
+// out over a cluster of 4 or 8 blocks: each scores its own heads, hands the scores to all blocks of the cluster through distributed shared
+// memory (mixing needs every head's score of a key), then mixes, weighs and sums up the values of its own heads.  Two tiles of 32 keys a
+// round, one pair of output numbers a thread; sums run in the order of the kernel above, tile by tile, and give its bits.
+// 32 heads on 8, chunks of 64, about 27 keys seen, us a call against the kernel above: bfloat16, heads of 128: 1 token 11.3 (in a model with
+// 64 keys 41 before), 32 tokens 16.2, 64 tokens 30.2 against 46.9; heads of 64: 10.9, 16.4, 17.1 against 32.0; float32, heads of 128: 64 tokens 34.1
+// against 68.9.  What is left is the chain: two cluster barriers, the rows of a page table, keys, values.
+constexpr int kFewTokens = 64;                 // 512 blocks: beyond it the clusters come in waves, while a block a token still fits one
+constexpr int kSpan = 2 * kTile;
+constexpr int kBatch = 16;                     // value rows a thread asks for before it uses the first
+
+template <typename T> struct RawPair { using type = float2; };
+template <> struct RawPair<__nv_bfloat16> { using type = __nv_bfloat162; };
+__device__ __forceinline__ float2 widen(float2 v) { return v; }
+__device__ __forceinline__ float2 widen(__nv_bfloat162 v) { return __bfloat1622float2(v); }
+
+// q . k over d numbers in order, eight 16-byte loads of the key row at a time (d is a multiple of 16 bytes' numbers).
+__device__ __forceinline__ float dot_ahead(const float* __restrict__ k, const float* __restrict__ q, int d) {
+    float acc = 0.f;
+    for (int i0 = 0; i0 < d; i0 += 32) {
+        float4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (i0 + 4 * u < d) v[u] = *reinterpret_cast<const float4*>(k + i0 + 4 * u);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (i0 + 4 * u < d) {
+                const float4 x = *reinterpret_cast<const float4*>(q + i0 + 4 * u);
+                acc = fmaf(v[u].x, x.x, acc);
+                acc = fmaf(v[u].y, x.y, acc);
+                acc = fmaf(v[u].z, x.z, acc);
+                acc = fmaf(v[u].w, x.w, acc);
+            }
+    }
+    return acc;
+}
+__device__ __forceinline__ float dot_ahead(const __nv_bfloat16* __restrict__ k, const float* __restrict__ q, int d) {
+    float acc = 0.f;
+    for (int i0 = 0; i0 < d; i0 += 64) {
+        uint4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (i0 + 8 * u < d) v[u] = *reinterpret_cast<const uint4*>(k + i0 + 8 * u);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (i0 + 8 * u < d) {
+                const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v[u]);
+                const float4 xa = *reinterpret_cast<const float4*>(q + i0 + 8 * u), xb = *reinterpret_cast<const float4*>(q + i0 + 8 * u + 4);
+                const float x[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 f = __bfloat1622float2(p[j]);
+                    acc = fmaf(f.x, x[2 * j], acc);
+                    acc = fmaf(f.y, x[2 * j + 1], acc);
+                }
+            }
+    }
+    return acc;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(512)
+talking_attn_few_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ cache, long long page_stride, long long v_off,
+                        const int* __restrict__ block_table, int table_width, const int* __restrict__ token_request,
+                        const int* __restrict__ positions, const float* __restrict__ talk, const float* __restrict__ slopes,
+                        T* __restrict__ out, int out_stride, int heads, int kv_heads, int dim, int vdim, int page_size, int chunk,
+                        float scale, int cluster) {
+    pdl_trigger();
+    extern __shared__ __align__(16) float smem[];
+    const int own = heads / cluster;                 // heads of this block
+    float* S = smem;                                 // [2][heads][kSpan] scores before mixing, written by all blocks of the cluster
+    float* A = S + 2 * heads * kSpan;                // [own][kSpan] mixed scores, then weights
+    float* talk_s = A + own * kSpan;                 // [heads (g)][own]
+    float* qs = talk_s + ((heads * own + 3) & ~3);   // [own][dim]
+    __shared__ long long row_base[kSpan];            // where a key's page starts, -1: the token does not see the key
+    __shared__ int row_off[kSpan];
+    __shared__ float tile_max[8][2], tile_sum[8][2], tile_corr[8][2], top[8];
+    const int rank = (int)llm_cluster_rank(), h0 = rank * own;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarp = blockDim.x >> 5, group = heads / kv_heads;
+    pdl_wait();
+    for (int i = tid; i < heads * own; i += blockDim.x) talk_s[i] = talk[(h0 + i % own) * heads + i / own];
+    if (tid < own) top[tid] = -INFINITY;
+    const int t = blockIdx.x / cluster;
+    const int pos = positions[t];
+    const int lo = chunk > 0 ? (pos / chunk) * chunk : 0;
+    const int* table = block_table + (size_t)token_request[t] * table_width;
+    for (int i = tid; i < own * dim; i += blockDim.x) qs[i] = to_f32(q[(size_t)t * q_stride + (size_t)h0 * dim + i]);
+    llm_cluster_sync();                              // every block runs before its shared memory is written
+
+    const int pairs = vdim / 2, mine = tid / pairs, d = 2 * (tid - mine * pairs);      // the thread's head and numbers of the output
+    const bool busy = mine < own;
+    const size_t v_head = (size_t)((h0 + (busy ? mine : 0)) / group) * page_size;
+    float2 acc = make_float2(0.f, 0.f);
+    float l = 0.f;
+    int buf = 0;
+    for (int k0 = lo & ~(kTile - 1); k0 <= pos; k0 += kSpan, buf ^= 1) {
+        float* Sb = S + buf * heads * kSpan;
+        if (tid < kSpan) {
+            const int j = k0 + tid;
+            const bool sees = j >= lo && j <= pos;
+            row_base[tid] = sees ? (long long)table[j / page_size] * page_stride : -1;
+            row_off[tid] = j % page_size;
+        }
+        __syncthreads();
+        for (int i = tid; i < own * kSpan; i += blockDim.x) {
+            const int hh = i / kSpan, jj = i % kSpan, g = h0 + hh;
+            float s = 0.f;
+            if (row_base[jj] >= 0)
+                s = scale * dot_ahead(cache + row_base[jj] + ((size_t)(g / group) * page_size + row_off[jj]) * dim, qs + hh * dim, dim) -
+                    slopes[g] * (float)(pos - k0 - jj);
+            for (int r = 0; r < cluster; ++r) llm_cluster_write(&Sb[g * kSpan + jj], r, s);
+        }
+        // the first values are on their way while the blocks meet
+        typename RawPair<T>::type raw[kBatch];
+        auto ask = [&](int first) {
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+                const long long base = row_base[first + u];
+                if (busy && base >= 0)
+                    raw[u] = *reinterpret_cast<const typename RawPair<T>::type*>(cache + base + v_off + (v_head + row_off[first + u]) * vdim + d);
+            }
+        };
+        ask(0);
+        llm_cluster_sync();                          // all heads' scores of the span are here
+        const int tiles = k0 + kTile <= pos ? 2 : 1;
+        for (int i = warp; i < 2 * own; i += nwarp) {
+            const int hh = i >> 1, jj = (i & 1) * kTile + lane;
+            float a = 0.f;
+            for (int g = 0; g < heads; ++g) a = fmaf(talk_s[g * own + hh], Sb[g * kSpan + jj], a);
+            a = row_base[jj] >= 0 ? a : -INFINITY;
+            A[hh * kSpan + jj] = a;
+            a = warp_max(a);
+            if (lane == 0) tile_max[hh][i & 1] = a;
+        }
+        __syncthreads();
+        for (int i = warp; i < tiles * own; i += nwarp) {
+            const int hh = tiles == 2 ? i >> 1 : i, tl = tiles == 2 ? i & 1 : 0, jj = tl * kTile + lane;
+            const float before = tl ? fmaxf(top[hh], tile_max[hh][0]) : top[hh], m = fmaxf(before, tile_max[hh][tl]);
+            const float p = row_base[jj] >= 0 ? expf(A[hh * kSpan + jj] - m) : 0.f;
+            A[hh * kSpan + jj] = p;
+            const float sum = warp_sum(p);
+            if (lane == 0) {
+                tile_sum[hh][tl] = sum;
+                tile_corr[hh][tl] = expf(before - m);      // 0 on the first tile
+            }
+        }
+        __syncthreads();
+        if (busy) {
+            for (int tl = 0; tl < tiles; ++tl) {
+                const float corr = tile_corr[mine][tl];
+                acc.x *= corr;
+                acc.y *= corr;
+                l = l * corr + tile_sum[mine][tl];
+#pragma unroll 1
+                for (int first = tl * kTile; first < (tl + 1) * kTile; first += kBatch) {
+                    if (first) ask(first);
+#pragma unroll
+                    for (int u = 0; u < kBatch; ++u) {
+                        const float p = A[mine * kSpan + first + u];
+                        if (p != 0.f) {
+                            const float2 x = widen(raw[u]);
+                            acc.x = fmaf(p, x.x, acc.x);
+                            acc.y = fmaf(p, x.y, acc.y);
+                        }
+                    }
+                }
+            }
+        }
+        if (tid < own) top[tid] = fmaxf(top[tid], tiles == 2 ? fmaxf(tile_max[tid][0], tile_max[tid][1]) : tile_max[tid][0]);
+        __syncthreads();                             // the span's tables are free
+    }
+    if (busy) {
+        const float inv = 1.0f / l;
+        store_pair(out + (size_t)t * out_stride + (size_t)(h0 + mine) * vdim + d, acc.x * inv, acc.y * inv);
+    }
+}
+
+// Blocks that share a token, 0: the kernel does not take these sizes.
+int few_cluster(int heads, int vdim) {
+    for (int c : {8, 4})
+        if (heads % c == 0 && heads / c <= 8 && heads / c * (vdim / 2) <= 512) return c;
+    return 0;
+}
+
+template <typename T>
+int launch_few(const void* q, int q_stride, const void* cache, long long page_stride, long long v_off, const int* block_table,
+               int table_width, const int* token_request, const int* positions, const float* talk, const float* slopes, void* out,
+               int out_stride, int tokens, int heads, int kv_heads, int dim, int vdim, int page_size, int chunk, float scale,
+               int cluster, cudaStream_t stream) {
+    const int own = heads / cluster;
+    int threads = (own * (vdim / 2) + 31) / 32 * 32;
+    if (threads < 128) threads = 128;
+    const size_t smem = sizeof(float) * (2 * (size_t)heads * kSpan + (size_t)own * kSpan + ((heads * own + 3) & ~3) + (size_t)own * dim);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(talking_attn_few_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    llm_launch_cluster(talking_attn_few_kernel<T>, (unsigned)(tokens * cluster), threads, smem, stream, (unsigned)cluster, (const T*)q, q_stride,
+                       (const T*)cache, page_stride, v_off, block_table, table_width, token_request, positions, talk, slopes, (T*)out,
+                       out_stride, heads, kv_heads, dim, vdim, page_size, chunk, scale, cluster);
+    LLM_CHECK_LAUNCH("talking_attention");
+    return 0;
+}
+
 template <typename T, int HPW>
 int launch_talking(const void* q, int q_stride, const void* cache, long long page_stride, long long v_off,
                    const int* block_table, int table_width, const int* token_request, const int* positions,
@@ -271,6 +474,10 @@ LLM_API int llm_talking_attention(const void* q, int q_stride, const void* cache
         // other's loads.  Few tokens (decoded ones): a warp for every head or two, since the block's own width is all the
         // parallelism there is.  (2,048 tokens, 32 heads of 64: 468 -> 381 us; 8 tokens: 78 against 96 us the other way round.)
         const bool many = tokens >= 2 * 148;
+        const int cluster = vec && tokens <= kFewTokens ? few_cluster(heads, vdim) : 0;
+        if (cluster && (size_t)(heads / cluster) * dim * sizeof(float) <= 64 * 1024)
+            return launch_few<T>(q, q_stride, cache, page_stride, v_off, block_table, table_width, token_request, positions, talk, slopes,
+                                 out, out_stride, tokens, heads, kv_heads, dim, vdim, page_size, chunk, scale, cluster, stream);
         if (heads <= 8) return LLM_TALK(1);
         if (heads <= 16) return many ? LLM_TALK(2) : LLM_TALK(1);
         if (heads <= 32) return many ? LLM_TALK(4) : LLM_TALK(2);

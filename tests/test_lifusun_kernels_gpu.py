@@ -144,6 +144,30 @@ def test_talking_attention_tiles_on_the_tensor_core(K, heads, kv_heads, dim, vdi
     close(out, one, torch.bfloat16, "against the one-token kernel")
 
 
+# a cluster a token (up to 64 tokens) against a block a token (more) and the restatement: one to eight heads a block, clusters of four and
+# eight, one tile and many rounds of two tiles, positions at, before and behind the edges of tiles, rounds and chunks, values of the lowest width
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,page,chunk", [(32, 8, 128, 128, 16, 64), (8, 4, 96, 80, 16, 48), (24, 8, 64, 64, 16, 0), (4, 4, 16, 8, 8, 24),
+                                                                (12, 3, 40, 256, 4, 100), (64, 8, 32, 128, 16, 0), (20, 5, 8, 16, 4, 8)])
+def test_talking_attention_of_few_tokens(K, dtype, heads, kv_heads, dim, vdim, page, chunk):
+    lengths = [1, 2, 31, 32, 33, 63, 64, 65, 96, 97, 127, 128, 129, 200, 47, 48, 49, 24, 25, 100, 101]
+    seqs = [(n, 1) for n in lengths + [150] * 50]
+    cache, meta, q = paged_case(dtype, heads, kv_heads, dim, vdim, page, seqs, seed=heads)
+    talk = (torch.eye(heads) + 0.3 * torch.randn(heads, heads, generator=torch.Generator().manual_seed(1))).to(DEV)
+    slopes = torch.tensor([2.0 ** (-8.0 * (h + 1) / heads) for h in range(heads)], device=DEV)
+    args = (heads, kv_heads, dim, vdim, chunk, dim ** -0.5)
+    many = torch.empty(q.shape[0], heads * vdim, device=DEV, dtype=dtype)
+    K.talking_attention(q, cache, meta, talk, slopes, many, *args)
+    want = R.ref_talking_attention(q, cache, meta.block_table, meta.token_request, meta.positions, talk, slopes, heads, kv_heads, dim, vdim,
+                                   page, chunk, dim ** -0.5)
+    n = len(lengths)
+    few = torch.full((n + 1, heads * vdim), 7.0, device=DEV, dtype=dtype)
+    part = SimpleNamespace(block_table=meta.block_table, token_request=meta.token_request[:n].contiguous(), positions=meta.positions[:n].contiguous())
+    K.talking_attention(q[:n].contiguous(), cache, part, talk, slopes, few[:n], *args)
+    close(few[:n], want[:n], dtype)
+    assert torch.equal(few[:n], many[:n]) and (few[n] == 7.0).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_talking_attention_edges_of_a_chunk(K, dtype):
     """The key just before a chunk's first position lines up with every query and would take all the weight if it were
