@@ -85,7 +85,7 @@ latent_prepare_kernel(const T* __restrict__ qd, int ld, const T* __restrict__ kv
 }
 
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(1024)
 headnorm_store_kernel(T* __restrict__ qkv, int ld, const float* __restrict__ q_gain, const float* __restrict__ k_gain, float eps,
                       T* __restrict__ cache, const int* __restrict__ slots, long long page_stride, int page_size, int heads,
                       int kv_heads, int dim, int vdim) {
@@ -263,7 +263,9 @@ LLM_API int llm_headnorm_store(void* qkv, int ld, const float* q_gain, const flo
     if (tokens == 0) return 0;
     return llm_dispatch_dtype(dtype, [&](auto tag) {
         using T = decltype(tag);
-        llm_launch(headnorm_store_kernel<T>, (unsigned)tokens, 128, 0, stream, (T*)qkv, ld, q_gain, k_gain, eps, (T*)cache, slots,
+        // few tokens: a warp a head instead of four warps that take the heads in turn
+        const int warps = tokens <= 148 ? (heads + kv_heads < 32 ? heads + kv_heads : 32) : 4;
+        llm_launch(headnorm_store_kernel<T>, (unsigned)tokens, warps < 4 ? 128 : warps * 32, 0, stream, (T*)qkv, ld, q_gain, k_gain, eps, (T*)cache, slots,
                    page_stride, page_size, heads, kv_heads, dim, vdim);
         LLM_CHECK_LAUNCH("headnorm_store");
         return 0;

@@ -5,6 +5,7 @@
 //                   One block per row, the row held in registers between the two passes, sums in a fixed order.
 //                   With a second gain the new residual row is normed as well, into rows of the engine's type: the norm
 //                   in front of the next sub-layer of a design that has norms on both sides of its sub-layers.
+//                   A branch may arrive as the k-split parts of a product (few rows only): they are added in split order as they are read.
 // llm_rmsnorm_rows: out[t] = in[t] * rsqrt(mean(in[t]^2) + eps) * weight for rows of the engine's type with strides of their
 //                   own (some columns of a wider product), float32 statistics.
 // llm_glu_clamped:  act = g * sigmoid(slope * g) * (u + 1) with g = min(gate, limit), u = clamp(up, -limit, limit),
@@ -76,6 +77,93 @@ norm_add_kernel(float* __restrict__ residual, const TB* __restrict__ branch, con
         next_out[row * width + i] = from_f32<TC>(res[i] * inv2 * to_f32(next_weight[i]));
 }
 
+// The same for few rows, when a row's time is what counts and not the rows in flight: 1024 threads a row, and everything a thread
+// will need is asked for at once (the gains even before the kernel ahead has finished) instead of in three dependent rounds of twelve loads.
+// The sums are those of the kernel above: 256 threads add the same numbers in the same order, out of shared memory.  One row of 3072 numbers took
+// 8.3 us there.  With the other kernels of few rows (token shift 21 us, head norms 11.7, wkv decays 13) and the product's parts read here instead of
+// added by a kernel ahead, a prompt of 1111 tokens and eight decode steps at the Rodapel 3B sizes went from 7.41 to 6.77 ms.
+constexpr int kFewThreads = 1024, kFewPer = 4, kFewWidth = kFewThreads * kFewPer;
+constexpr int kFewRows = 148;        // a block is a row and half an SM: beyond a wave of SMs the small blocks are as fast
+
+template <typename TB, typename TW, typename TC>
+__global__ void __launch_bounds__(kFewThreads)
+norm_add_few_kernel(float* __restrict__ residual, const TB* __restrict__ branch, const TW* __restrict__ weight, TC* __restrict__ cast,
+                    int width, float eps, int accumulate, const TW* __restrict__ next_weight, TC* __restrict__ next_out, int splits,
+                    size_t split_stride) {
+    pdl_trigger();
+    extern __shared__ float row_buf[];       // width floats
+    __shared__ float red[kNormThreads / 32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const size_t row = blockIdx.x;
+    float b[kFewPer], w[kFewPer], nw[kFewPer], r[kFewPer];
+#pragma unroll
+    for (int j = 0; j < kFewPer; ++j) {
+        const int i = tid + j * kFewThreads;
+        w[j] = i < width ? to_f32(weight[i]) : 0.f;
+        nw[j] = next_out && i < width ? to_f32(next_weight[i]) : 0.f;
+    }
+    pdl_wait();
+#pragma unroll
+    for (int j = 0; j < kFewPer; ++j) {
+        const int i = tid + j * kFewThreads;
+        r[j] = accumulate && i < width ? residual[row * width + i] : 0.f;
+        if (splits == 0) b[j] = i < width ? to_f32(branch[row * width + i]) : 0.f;
+    }
+    if (splits > 0) {
+        const float* parts = reinterpret_cast<const float*>(branch) + row * width;
+        float e[kFewPer][kMaxParts];
+#pragma unroll
+        for (int j = 0; j < kFewPer; ++j)
+#pragma unroll
+            for (int k = 0; k < kMaxParts; ++k)
+                if (k < splits && tid + j * kFewThreads < width) e[j][k] = parts[k * split_stride + tid + j * kFewThreads];
+#pragma unroll
+        for (int j = 0; j < kFewPer; ++j) {
+            b[j] = tid + j * kFewThreads < width ? e[j][0] : 0.f;
+#pragma unroll
+            for (int k = 1; k < kMaxParts; ++k)
+                if (k < splits && tid + j * kFewThreads < width) b[j] += e[j][k];
+        }
+    }
+    // sums of squares as kNormThreads threads take them: element tid + kNormThreads * j, from round `from` to the row's end, then from 0
+    auto square_sum = [&](int from) {
+        float ss = 0.f;
+        if (warp < kNormThreads / 32) {
+            for (int i = tid + from * kNormThreads; i < width; i += kNormThreads) ss += row_buf[i] * row_buf[i];
+            for (int i = tid; i < width && i < from * kNormThreads; i += kNormThreads) ss += row_buf[i] * row_buf[i];
+            ss = warp_sum(ss);
+            if (lane == 0) red[warp] = ss;
+        }
+        __syncthreads();
+        return warp_sum(lane < kNormThreads / 32 ? red[lane] : 0.f);
+    };
+#pragma unroll
+    for (int j = 0; j < kFewPer; ++j)
+        if (tid + j * kFewThreads < width) row_buf[tid + j * kFewThreads] = b[j];
+    __syncthreads();
+    const float inv = 1.0f / sqrtf(square_sum(0) / (float)width + eps);
+#pragma unroll
+    for (int j = 0; j < kFewPer; ++j) {
+        const int i = tid + j * kFewThreads;
+        if (i < width) {
+            float y = b[j] * inv * w[j];
+            if (accumulate) y += r[j];
+            b[j] = y;
+            residual[row * width + i] = y;
+            if (cast) cast[row * width + i] = from_f32<TC>(y);
+            if (next_out) row_buf[i] = y;
+        }
+    }
+    if (!next_out) return;                 // the same for the whole block
+    __syncthreads();
+    const float inv2 = 1.0f / sqrtf(square_sum(kNormPer) / (float)width + eps);
+#pragma unroll
+    for (int j = 0; j < kFewPer; ++j) {
+        const int i = tid + j * kFewThreads;
+        if (i < width) next_out[row * width + i] = from_f32<TC>(b[j] * inv2 * nw[j]);
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(128)
 rmsnorm_rows_kernel(const T* __restrict__ in, long long ld_in, T* __restrict__ out, long long ld_out, const float* __restrict__ weight,
@@ -107,28 +195,60 @@ __global__ void glu_act_kernel(const T* __restrict__ gu, T* __restrict__ act, in
     }
 }
 
+// Eight neighbouring numbers a thread where `vec` (rows and their halves start on 16 bytes), else one.  (A division of 64 bits for every
+// number and one number a load: 1111 rows of 8192 took 33 us.)
 template <typename T>
-__global__ void glu_clamped_kernel(const T* __restrict__ gu, T* __restrict__ act, int tokens, int inner, float limit, float slope) {
+__global__ void __launch_bounds__(256)
+glu_clamped_kernel(const T* __restrict__ gu, T* __restrict__ act, int tokens, int inner, float limit, float slope, int vec) {
     pdl_trigger();
     pdl_wait();
-    const size_t n = (size_t)tokens * inner;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t t = i / inner, c = i % inner;
-        const float g = fminf(to_f32(gu[t * 2 * inner + c]), limit);
-        const float u = fminf(fmaxf(to_f32(gu[t * 2 * inner + inner + c]), -limit), limit);
-        act[i] = from_f32<T>(g / (1.0f + expf(-slope * g)) * (u + 1.0f));
+    auto f = [&](float g, float u) {
+        g = fminf(g, limit);
+        u = fminf(fmaxf(u, -limit), limit);
+        return g / (1.0f + expf(-slope * g)) * (u + 1.0f);
+    };
+    for (int t = blockIdx.y; t < tokens; t += gridDim.y) {
+        const T* gr = gu + (size_t)t * 2 * inner;
+        T* ar = act + (size_t)t * inner;
+        const int first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+        if (vec) {
+            constexpr int kPieces = sizeof(T) / 2;           // 16-byte loads of eight numbers
+            for (int c = first; c < inner / 8; c += step) {
+                uint4 g[kPieces], u[kPieces], a[kPieces];
+#pragma unroll
+                for (int e = 0; e < kPieces; ++e) {
+                    g[e] = reinterpret_cast<const uint4*>(gr + 8 * c)[e];
+                    u[e] = reinterpret_cast<const uint4*>(gr + inner + 8 * c)[e];
+                }
+                const T *gp = reinterpret_cast<const T*>(g), *up = reinterpret_cast<const T*>(u);
+                T* ap = reinterpret_cast<T*>(a);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) ap[e] = from_f32<T>(f(to_f32(gp[e]), to_f32(up[e])));
+#pragma unroll
+                for (int e = 0; e < kPieces; ++e) reinterpret_cast<uint4*>(ar + 8 * c)[e] = a[e];
+            }
+        } else {
+            for (int c = first; c < inner; c += step) ar[c] = from_f32<T>(f(to_f32(gr[c]), to_f32(gr[inner + c])));
+        }
     }
 }
 
 }  // namespace
 
+// Rows up to which llm_norm_add takes the parts of a product (width up to 4096).
+LLM_API int llm_norm_add_few_rows(int width) { return width <= kFewWidth ? kFewRows : 0; }
+
 // branch [tokens, width] of `branch_dtype`; weight float32 or bfloat16 (`weight_dtype`); cast: null or [tokens, width] of
-// `cast_dtype`.  accumulate == 0 writes the normed row instead of adding it (an embedding's norm).
+// `cast_dtype`.  accumulate == 0 writes the normed row instead of adding it (an embedding's norm).  splits > 0: `branch` is float32 parts
+// [splits][tokens][width], `split_stride` numbers apart (at most llm_norm_add_few_rows() rows, of at most 4096 numbers).
 LLM_API int llm_norm_add(float* residual, const void* branch, int branch_dtype, const void* weight, int weight_dtype,
                          void* cast, int cast_dtype, int tokens, int width, float eps, int accumulate, const void* next_weight,
-                         void* next_out, cudaStream_t stream) {
+                         void* next_out, int splits, long long split_stride, cudaStream_t stream) {
     if (tokens == 0) return 0;
     if (width <= 0) LLM_FAIL(-1, "norm_add: width %d", width);
+    const bool few = tokens <= kFewRows && width <= kFewWidth;
+    if (splits < 0 || splits > kMaxParts || (splits > 0 && (!few || branch_dtype != LLM_F32)))
+        LLM_FAIL(-1, "norm_add: %d parts of %d rows of %d numbers are not taken", splits, tokens, width);
     if ((next_weight == nullptr) != (next_out == nullptr)) LLM_FAIL(-1, "norm_add: the second norm needs a gain and a place for its rows");
     return llm_dispatch_dtype(branch_dtype, [&](auto tb) {
         using TB = decltype(tb);
@@ -136,8 +256,13 @@ LLM_API int llm_norm_add(float* residual, const void* branch, int branch_dtype, 
             using TW = decltype(tw);
             return llm_dispatch_dtype(cast || next_out ? cast_dtype : LLM_BF16, [&](auto tc) {
                 using TC = decltype(tc);
-                llm_launch(norm_add_kernel<TB, TW, TC>, (unsigned)tokens, kNormThreads, 0, stream, residual, (const TB*)branch,
-                           (const TW*)weight, (TC*)cast, width, eps, accumulate, (const TW*)next_weight, (TC*)next_out);
+                if (few)
+                    llm_launch(norm_add_few_kernel<TB, TW, TC>, (unsigned)tokens, kFewThreads, sizeof(float) * width, stream, residual,
+                               (const TB*)branch, (const TW*)weight, (TC*)cast, width, eps, accumulate, (const TW*)next_weight, (TC*)next_out,
+                               splits, (size_t)split_stride);
+                else
+                    llm_launch(norm_add_kernel<TB, TW, TC>, (unsigned)tokens, kNormThreads, 0, stream, residual, (const TB*)branch,
+                               (const TW*)weight, (TC*)cast, width, eps, accumulate, (const TW*)next_weight, (TC*)next_out);
                 LLM_CHECK_LAUNCH("norm_add");
                 return 0;
             });
@@ -175,11 +300,12 @@ LLM_API int llm_glu_act(const void* gu, void* act, int dtype, int tokens, int in
 LLM_API int llm_glu_clamped(const void* gu, void* act, int dtype, int tokens, int inner, float limit, float slope,
                             cudaStream_t stream) {
     if (tokens == 0 || inner == 0) return 0;
-    const size_t n = (size_t)tokens * inner;
-    const unsigned blocks = (unsigned)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
+    const int vec = inner % 8 == 0 && !(((uintptr_t)gu | (uintptr_t)act) & 15);
+    const int work = vec ? inner / 8 : inner, threads = work < 256 ? (work + 31) / 32 * 32 : 256;
+    const dim3 grid((work + threads - 1) / threads, tokens < 65535 ? tokens : 65535);
     return llm_dispatch_dtype(dtype, [&](auto tag) {
         using T = decltype(tag);
-        llm_launch(glu_clamped_kernel<T>, blocks, 256, 0, stream, (const T*)gu, (T*)act, tokens, inner, limit, slope);
+        llm_launch(glu_clamped_kernel<T>, grid, threads, 0, stream, (const T*)gu, (T*)act, tokens, inner, limit, slope, vec);
         LLM_CHECK_LAUNCH("glu_clamped");
         return 0;
     });

@@ -21,7 +21,7 @@ __global__ void embed_kernel(const int* __restrict__ ids, const TW* __restrict__
     const bool ok = id >= 0 && id < vocab;  // the host refuses such ids; never read out of range
     const TW* src = table + (size_t)(ok ? id : 0) * width;
     float* dst = out + (size_t)t * width;
-    for (int i = threadIdx.x; i < width; i += blockDim.x) dst[i] = ok ? scale * to_f32(src[i]) : 0.f;
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < width; i += gridDim.y * blockDim.x) dst[i] = ok ? scale * to_f32(src[i]) : 0.f;
 }
 
 LLM_API int llm_embed(const int* ids, const void* table, int table_dtype, float* out, int tokens,
@@ -29,7 +29,10 @@ LLM_API int llm_embed(const int* ids, const void* table, int table_dtype, float*
     if (tokens == 0) return 0;
     return llm_dispatch_dtype(table_dtype, [&](auto tag) {
         using TW = decltype(tag);
-        llm_launch(embed_kernel<TW>, tokens, 256, 0, stream, ids, (const TW*)table, out, width, vocab, scale);
+        // few tokens: a number a thread, a row over several blocks
+        const int pieces = tokens <= 64 ? (width + 255) / 256 : 1;
+        llm_launch(embed_kernel<TW>, dim3(tokens, pieces < 65535 ? pieces : 65535), 256, 0, stream, ids, (const TW*)table, out, width, vocab,
+                   scale);
         LLM_CHECK_LAUNCH("embed");
         return 0;
     });

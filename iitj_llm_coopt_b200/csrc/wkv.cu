@@ -29,7 +29,7 @@ token_shift_kernel(const T* __restrict__ x, const float* __restrict__ mu, const 
     const int b = token_request[t];
     const bool first = t == cu_seqlens[b];
     const float* prev_state = before + (size_t)state_slots[b] * width;
-    for (int c = threadIdx.x; c < width; c += blockDim.x) {
+    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < width; c += gridDim.y * blockDim.x) {
         const float v = to_f32(x[(size_t)t * width + c]);
         const float p = first ? prev_state[c] : to_f32(x[(size_t)(t - 1) * width + c]);
         for (int s = 0; s < streams; ++s)
@@ -85,6 +85,45 @@ wkv_decay_kernel(const float* __restrict__ low, const float* __restrict__ w2, co
 #pragma unroll
     for (int t = 0; t < kDecayTokens; ++t)
         if (t < live) out[(size_t)(t0 + t) * channels + c] = expf(-expf(acc[t] + base));
+}
+
+// Few tokens: a channel a thread, its row of W2 asked for while the kernel ahead finishes, 64 channels a block.  The sum over j in order, as above.
+// (The kernel above stages W2 piece by piece behind barriers: one token of 3072 channels and rank 64 took 13 us.)
+constexpr int kFewTokens = 32, kFewChannels = 64, kFewAhead = 8;       // kFewAhead: loads of 16 bytes in flight
+
+__global__ void __launch_bounds__(kFewChannels)
+wkv_decay_few_kernel(const float* __restrict__ low, const float* __restrict__ w2, const float* __restrict__ w0, float* __restrict__ out,
+                     int channels, int rank) {
+    extern __shared__ __align__(16) float th_row[];          // [rank]
+    pdl_trigger();
+    const int t = blockIdx.x, c = blockIdx.y * kFewChannels + threadIdx.x;
+    const bool live = c < channels;
+    const float* w = w2 + (size_t)(live ? c : 0) * rank;
+    float4 v[kFewAhead];
+    auto ask = [&](int j0) {
+#pragma unroll
+        for (int u = 0; u < kFewAhead; ++u)
+            if (j0 + 4 * u < rank) v[u] = *reinterpret_cast<const float4*>(w + j0 + 4 * u);
+    };
+    ask(0);
+    const float base = live ? w0[c] : 0.f;
+    pdl_wait();
+    for (int j = threadIdx.x; j < rank; j += kFewChannels) th_row[j] = tanhf(low[(size_t)t * rank + j]);
+    __syncthreads();
+    float acc = 0.f;
+    for (int j0 = 0; j0 < rank; j0 += 4 * kFewAhead) {
+        if (j0) ask(j0);
+#pragma unroll
+        for (int u = 0; u < kFewAhead; ++u)
+            if (j0 + 4 * u < rank) {
+                const float4 x = *reinterpret_cast<const float4*>(th_row + j0 + 4 * u);
+                acc = fmaf(v[u].x, x.x, acc);
+                acc = fmaf(v[u].y, x.y, acc);
+                acc = fmaf(v[u].z, x.z, acc);
+                acc = fmaf(v[u].w, x.w, acc);
+            }
+    }
+    if (live) out[(size_t)t * channels + c] = expf(-expf(acc + base));
 }
 
 template <typename T, int DMAX>
@@ -196,7 +235,9 @@ LLM_API int llm_token_shift(const void* x, const float* mu, const float* before,
     if (tokens == 0) return 0;
     return llm_dispatch_dtype(dtype, [&](auto tag) {
         using T = decltype(tag);
-        llm_launch(token_shift_kernel<T>, (unsigned)tokens, 256, 0, stream, (const T*)x, mu, before, state_slots, token_request,
+        // few tokens: a channel a thread, a row's channels over several blocks
+        const int pieces = tokens <= kFewTokens ? (width + 255) / 256 : 1;
+        llm_launch(token_shift_kernel<T>, dim3((unsigned)tokens, pieces < 65535 ? pieces : 65535), 256, 0, stream, (const T*)x, mu, before, state_slots, token_request,
                    cu_seqlens, (T*)out, tokens, width, streams);
         LLM_CHECK_LAUNCH("token_shift");
         return 0;
@@ -206,6 +247,13 @@ LLM_API int llm_token_shift(const void* x, const float* mu, const float* before,
 LLM_API int llm_wkv_decay(const float* low, const float* w2, const float* w0, float* out, int tokens, int channels, int rank,
                           cudaStream_t stream) {
     if (tokens == 0) return 0;
+    // (rows of W2 that start on 16 bytes; a rank whose row fits shared memory without asking)
+    const int few_blocks = (channels + kFewChannels - 1) / kFewChannels;
+    if (tokens <= kFewTokens && rank % 4 == 0 && rank <= 8192 && !((uintptr_t)w2 & 15) && few_blocks <= 65535) {
+        llm_launch(wkv_decay_few_kernel, dim3((unsigned)tokens, few_blocks), kFewChannels, sizeof(float) * rank, stream, low, w2, w0, out, channels, rank);
+        LLM_CHECK_LAUNCH("wkv_decay");
+        return 0;
+    }
     const int c_blocks = (channels + kDecayThreads - 1) / kDecayThreads;
     if (c_blocks > 65535) LLM_FAIL(-1, "wkv_decay: %d channels are too many for one launch", channels);
     llm_launch(wkv_decay_kernel, dim3((unsigned)((tokens + kDecayTokens - 1) / kDecayTokens), c_blocks), kDecayThreads, 0, stream, low, w2, w0, out,

@@ -113,7 +113,8 @@ _SIGNATURES = {
     "llm_retention_headnorm_gate": [_c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_float,
                                     _c_void_p],
     "llm_norm_add": [_c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_float, _c_int, _c_void_p,
-                     _c_void_p, _c_void_p],
+                     _c_void_p, _c_int, ctypes.c_longlong, _c_void_p],
+    "llm_norm_add_few_rows": [_c_int],
     "llm_add_dynamic_tanh": [_c_void_p, _c_void_p, _c_int, _c_int, ctypes.c_longlong, _c_void_p, _c_void_p, _c_int, _c_float, _c_void_p,
                              _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, ctypes.c_longlong, _c_int, _c_int, _c_int, _c_void_p],
     "llm_add_branch_rmsnorm": [_c_void_p, _c_void_p, _c_int, _c_int, ctypes.c_longlong, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int,
@@ -1003,11 +1004,17 @@ class Kernels:
     def norm_add(self, residual, branch, weight, eps, cast_out=None, accumulate: bool = True, next_weight=None, next_out=None):
         """residual (+)= rmsnorm(branch) * weight with float32 statistics (csrc/branch_norm.cu); `cast_out`: a copy of the new
         residual in another type (what the next sub-layer reads).  `accumulate` False writes the normed rows instead.
-        With `next_weight` and `next_out` the new residual rows are normed too: next_out = rmsnorm(residual) * next_weight."""
+        With `next_weight` and `next_out` the new residual rows are normed too: next_out = rmsnorm(residual) * next_weight.
+        `branch` may be a PartialSums: the parts of few rows are added while they are read."""
         _check(residual, "norm_add.residual", torch.float32, 2)
+        tokens, width = residual.shape
+        splits, stride = 0, 0
+        if isinstance(branch, PartialSums) and branch.splits <= 8 and tokens <= self.lib.llm_norm_add_few_rows(width):
+            _need(tuple(branch.shape) == (tokens, width), "norm_add: shapes differ")
+            splits, stride, branch = branch.splits, branch.stride, branch.parts[0]
+        branch = materialize(branch)
         _check(branch, "norm_add.branch", tuple(DTYPE_CODE), 2)
         _check(weight, "norm_add.weight", tuple(DTYPE_CODE), 1)
-        tokens, width = residual.shape
         _need(tuple(branch.shape) == (tokens, width) and weight.shape[0] == width, "norm_add: shapes differ")
         if cast_out is not None:
             _check(cast_out, "norm_add.cast_out", tuple(DTYPE_CODE), 2)
@@ -1022,7 +1029,7 @@ class Kernels:
             _need(next_weight is None, "norm_add: a second gain without a place for its rows")
         self._call("llm_norm_add", _ptr(residual), _ptr(branch), DTYPE_CODE[branch.dtype], _ptr(weight), DTYPE_CODE[weight.dtype],
                    _ptr(cast_out), DTYPE_CODE[typed.dtype] if typed is not None else 0, tokens, width, float(eps),
-                   1 if accumulate else 0, _ptr(next_weight), _ptr(next_out), self._stream())
+                   1 if accumulate else 0, _ptr(next_weight), _ptr(next_out), splits, stride, self._stream())
         return residual
 
     def rmsnorm_rows(self, x, weight, eps, out):

@@ -17,8 +17,13 @@ Nothing is left over for the next layer, so its delta is None.
 """
 from __future__ import annotations
 
-from ..kernels import materialize
+from ..kernels import PartialSums, materialize
 from .base import delta_for
+
+
+def _rows_or_parts(branch):
+    """A branch as `Kernels.norm_add` takes it: a tensor, or the parts of a product."""
+    return branch if isinstance(branch, PartialSums) else materialize(branch)
 
 
 class Arrangement:
@@ -97,7 +102,7 @@ class BranchNormBlock(Arrangement):
     def _add_branch(self, ctx, residual, branch, norm):
         dtype = self.mixer.dtype
         cast = None if dtype == residual.dtype else ctx.buffer(self.CAST, tuple(residual.shape), dtype)
-        norm.k.norm_add(residual, materialize(branch), norm.weight, norm.eps, cast_out=cast)
+        norm.k.norm_add(residual, _rows_or_parts(branch), norm.weight, norm.eps, cast_out=cast)
         if cast is not None:
             ctx.shared[self.CAST] = cast
         return residual if cast is None else cast
@@ -139,7 +144,7 @@ class SandwichBlock(Arrangement):
         cast = None
         if side is not None and self.mixer.dtype != residual.dtype:
             cast = ctx.buffer(self.CAST, tuple(residual.shape), self.mixer.dtype)
-        norm.k.norm_add(residual, materialize(branch), norm.weight, norm.eps, cast_out=cast)
+        norm.k.norm_add(residual, _rows_or_parts(branch), norm.weight, norm.eps, cast_out=cast)
         ctx.shared.pop(self.CAST, None)
         if side is not None:
             side.forward(ctx, residual, residual if cast is None else cast)
@@ -154,7 +159,7 @@ class SandwichBlock(Arrangement):
         a = self.mixer.forward(ctx, self._enter(ctx, residual, delta), call)
         post, front = self.mixer_post_norm, self.feed_forward_norm
         x = ctx.buffer(f"norm.{front.part_name}.out", tuple(residual.shape), self.mixer.dtype)
-        post.k.norm_add(residual, materialize(a), post.weight, post.eps, next_weight=front.weight, next_out=x)
+        post.k.norm_add(residual, _rows_or_parts(a), post.weight, post.eps, next_weight=front.weight, next_out=x)
         self._last_add(ctx, residual, self.feed_forward.forward(ctx, x), self.feed_forward_post_norm)
         return residual, None
 

@@ -60,7 +60,7 @@ class GLU(Part):
             self.k.linear(x, self.gate_up, gu)
             self.k.glu_act(gu, act, self.activation)
         out = ctx.buffer("ffn.out", (t, self.width), self.dtype)
-        return self.k.linear(act, self.down, out)
+        return self.k.linear(act, self.down, out, defer=True)
 
 
 class ClampedGLU(Part):
@@ -91,7 +91,7 @@ class ClampedGLU(Part):
         act = ctx.buffer("ffn.act", (t, self.inner), self.dtype)
         self.k.glu_clamped(gu, act, self.limit, self.slope)
         out = ctx.buffer("ffn.out", (t, self.width), self.dtype)
-        return self.k.linear(act, self.down, out)
+        return self.k.linear(act, self.down, out, defer=True)
 
 
 class PolyNormMLP(Part):
@@ -122,7 +122,7 @@ class PolyNormMLP(Part):
         act = ctx.buffer("ffn.act", (t, self.inner), self.dtype)
         self.k.poly_norm(z, self.act, self.eps, act)
         out = ctx.buffer("ffn.out", (t, self.width), self.dtype)
-        return self.k.linear(act, self.down, out)
+        return self.k.linear(act, self.down, out, defer=True)
 
 
 class RoutedGLU(Part):

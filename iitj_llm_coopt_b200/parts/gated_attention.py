@@ -162,4 +162,4 @@ class GatedAttention(Part):
         self.k.attention_flat(qkv, view, meta, attn, self.heads, self.kv_heads, self.head_dim, self.value_dim,
                               window=self.window, scale=self.scale, gate=gate, plan=ctx.prepared.get(self.prepare_key), **self.extras)
         out = ctx.buffer("attn.out", (t, self.width), self.dtype)
-        return self.k.linear(attn, self.o, out)
+        return self.k.linear(attn, self.o, out, defer=True)

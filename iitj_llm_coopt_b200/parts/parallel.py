@@ -13,6 +13,7 @@ import dataclasses
 
 import torch
 
+from ..kernels import materialize
 from .base import ParamSpec, Part
 
 SIDES = ("left", "right")
@@ -76,7 +77,7 @@ class ParallelMixer(Part):
         if call.state is None:
             raise ValueError("parallel mixer: the right side needs a cache entry of its own (LayerCall.state)")
         self.left.part_name, self.right.part_name = self.part_name + ".left", self.part_name + ".right"
-        a = self.left.forward(ctx, x, call)
-        b = self.right.forward(ctx, x, dataclasses.replace(call, cache=call.state, state=None))
+        a = materialize(self.left.forward(ctx, x, call))      # (parts of its product would not outlive the right side's products)
+        b = materialize(self.right.forward(ctx, x, dataclasses.replace(call, cache=call.state, state=None)))
         out = ctx.buffer("parallel.out", (x.shape[0], self.width), torch.float32)
         return self.k.branch_mean([a, b], [self.left_gain, self.right_gain], self.scale, self.eps, out)

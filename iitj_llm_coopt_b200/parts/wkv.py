@@ -77,4 +77,4 @@ class WKV(Part):
         self.k.wkv_scan(rkvg, decay, self.u, self.norm, self.eps, state, ctx.state_slots, ctx.cu_seqlens, gated,
                         self.heads, self.head_dim, write=call.write, last_rows=(x, before) if call.write else None)
         out = ctx.buffer("attn.out", (t, self.width), self.dtype)
-        return self.k.linear(gated, self.o, out)
+        return self.k.linear(gated, self.o, out, defer=True)

@@ -338,3 +338,41 @@ def test_planted_keys_at_the_window_s_edges(K, dtype, window, page, total):
             close(out, want, dtype)
         if window:
             assert (want[:, :vdim].amax(1) > 1.0).any()       # the planted value shows in the answer
+
+
+# few rows (a block of 1024 threads a row, the parts of a product added as they are read) against many (256 threads a row) and the
+# restatement: one thread's number, the edges of the rounds of 256 and 1024, the widest row that few rows take, one more
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tokens,width,splits", [(1, 8, 2), (3, 1024, 8), (148, 1028, 3), (2, 2052, 5), (5, 3072, 1), (1, 4096, 8), (2, 4100, 4), (149, 512, 2)])
+def test_norm_add_of_parts(K, dtype, tokens, width, splits):
+    from iitj_llm_coopt_b200.kernels import PartialSums
+    g = torch.Generator(device="cuda").manual_seed(width)
+    rnd = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
+    parts, w, w2, res = rnd(splits, tokens, width), rnd(width), rnd(width), rnd(tokens, width)
+    total = parts[0].clone()
+    for p in parts[1:]:
+        total += p
+    for accumulate in (True, False):
+        got, cast, nxt = res.clone(), torch.empty(tokens, width, device="cuda", dtype=dtype), torch.empty(tokens, width, device="cuda", dtype=dtype)
+        K.norm_add(got, PartialSums(K, parts, torch.empty_like(total)), w, 1e-5, cast_out=cast, accumulate=accumulate, next_weight=w2, next_out=nxt)
+        want = R.ref_norm_add(res, total, w, 1e-5, accumulate)
+        assert ((got - want).norm() / want.norm()).item() < 1e-6          # (two sums of `width` numbers in float32)
+        assert torch.equal(cast, got.to(dtype))
+        unit = got.double() * torch.rsqrt(got.double().pow(2).mean(1, keepdim=True) + 1e-5) * w2
+        assert ((nxt - unit).norm() / unit.norm()).item() < (1e-6 if dtype == torch.float32 else 2.0 ** -8)
+        rows = 160                                                          # the same rows among many: the same bits
+        if tokens < rows and width <= 4096:
+            many, big = res.repeat(rows, 1)[:rows].contiguous(), total.repeat(rows, 1)[:rows].contiguous()
+            K.norm_add(many, big, w, 1e-5, accumulate=accumulate)
+            assert torch.equal(many[:tokens], got)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tokens,inner", [(1, 8), (3, 100), (2, 2056), (70, 8192)])
+def test_glu_clamped_pieces(K, dtype, tokens, inner):
+    gu = (2.0 * torch.randn(tokens, 2 * inner, generator=torch.Generator(device="cuda").manual_seed(inner), device="cuda")).to(dtype)
+    out = torch.empty(tokens, inner, device="cuda", dtype=dtype)
+    K.glu_clamped(gu, out, 1.5, 1.7)
+    gate, up = gu[:, :inner].double().clamp(max=1.5), gu[:, inner:].double().clamp(-1.5, 1.5)
+    want = gate * torch.sigmoid(1.7 * gate) * (up + 1.0)
+    assert ((out - want).norm() / want.norm()).item() < (1e-6 if dtype == torch.float32 else 2.0 ** -8)
