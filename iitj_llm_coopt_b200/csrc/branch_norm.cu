@@ -146,8 +146,8 @@ norm_add_few_kernel(float* __restrict__ residual, const TB* __restrict__ branch,
     for (int j = 0; j < kFewPer; ++j) {
         const int i = tid + j * kFewThreads;
         if (i < width) {
-            float y = b[j] * inv * w[j];
-            if (accumulate) y += r[j];
+            const float scaled = b[j] * inv;
+            const float y = accumulate ? fmaf(scaled, w[j], r[j]) : scaled * w[j];
             b[j] = y;
             residual[row * width + i] = y;
             if (cast) cast[row * width + i] = from_f32<TC>(y);
