@@ -1292,6 +1292,12 @@ class Kernels:
         """Neighbouring tokens of one request that a block of the tensor-core attention over flat pages takes."""
         return 64 // self.lib.llm_attention_flat_mma_heads_per_block(heads, kv_heads)
 
+    def flat_f32_runs(self, heads: int, kv_heads: int, key_dim: int, value_dim: int, shared_value: bool) -> int:
+        """Neighbouring tokens of one request that a block of the float32 tile kernel (csrc/attention_f32.cu) takes, 0 where it does not
+        serve attention over flat pages: its pages are a key plane and a value plane of one size, which is what flat pages are when keys
+        and values have one size and values of their own."""
+        return 64 if key_dim == value_dim and not shared_value and self.lib.llm_attention_f32_supported(heads, kv_heads, key_dim) else 0
+
     def flat_key_splits(self, requests: int, heads: int, kv_heads: int, key_dim: int, value_dim: int, shared_value: bool,
                         longest: int) -> int:
         """Over how many blocks the keys of each decoded token are shared out: as many as fill the SMs once with the blocks an
@@ -1353,6 +1359,23 @@ class Kernels:
             if splits > 1:
                 self.launches += 1      # the merge kernel
             return out
+        if q.dtype == torch.float32 and plan is not None and tokens <= 65535 and q.shape[1] % 4 == 0 and \
+                self.flat_f32_runs(heads, kv_heads, key_dim, value_dim, shared_value) and \
+                gate is None and slopes is None and sinks is None and every == 0 and softcap == 0 and \
+                not (q.data_ptr() | out.data_ptr() | cache_layer.data_ptr()) & 15:
+            # plain scores over planes of one size: the kernels of float32 attention, whose sums are the general kernel's, in its order (a
+            # token behind 337 keys, 32 heads on 8 of 64 numbers, took 200 us there: one warp walks all keys of a head)
+            if getattr(plan, "single", False):
+                self._call("llm_attention_f32_single", _ptr(q), q.shape[1], _ptr(cache_layer), _ptr(meta.block_table),
+                           meta.block_table.shape[1], None, tokens, _ptr(meta.token_request), _ptr(meta.positions), _ptr(out),
+                           out.shape[1], heads, kv_heads, key_dim, page_size, int(window), float(scale), self._stream())
+                return out
+            runs = plan.device_arrays.get("runs")
+            if runs is not None:
+                self._call("llm_attention_f32_tiles", _ptr(q), q.shape[1], _ptr(cache_layer), _ptr(meta.block_table),
+                           meta.block_table.shape[1], _ptr(runs), runs.shape[0] // 4, _ptr(out), out.shape[1], heads, kv_heads, key_dim,
+                           page_size, int(window), float(scale), self._stream())
+                return out
         self._call("llm_attention_flat", _ptr(q), q.shape[1], _ptr(cache_layer), cache_layer.shape[1], _ptr(meta.block_table),
                    meta.block_table.shape[1], _ptr(meta.token_request), _ptr(meta.positions), _ptr(gate), gate_cols, _ptr(out),
                    out.shape[1], DTYPE_CODE[q.dtype], tokens, heads, kv_heads, key_dim, value_dim, 1 if shared_value else 0, page_size,

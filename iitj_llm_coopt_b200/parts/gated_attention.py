@@ -123,7 +123,7 @@ class GatedAttention(Part):
         return (self.position,) if self.position is not None else ()
 
     def prepare_step(self, shape):
-        return plan_flat_tiles(self.k, shape, self.heads, self.kv_heads, self.head_dim, self.value_dim, self.window)
+        return plan_flat_tiles(self.k, shape, self.heads, self.kv_heads, self.head_dim, self.value_dim, self.window, dtype=self.dtype)
 
     def load(self, tensors: dict) -> None:
         super().load(tensors)
