@@ -32,7 +32,7 @@
 //
 // What bounds it: a decode step the HBM bytes of W, a prompt the tensor cores at seven bfloat16 products per float32 product (six of
 // them of use: 278 TFLOP/s of the measured bf16 rate) and the barriers above.  Measured with the planes, cold weights, against the
-// product on the CUDA cores (gemm_f32.cu): 5 tokens, 2048 x 2048 195 -> 10 us, 2048 x 8192 770 -> 34 us; one token, 128256 x 2048
+// product on the CUDA cores (gemm_f32.cu): 5 tokens, 2048 x 2048 195 -> 10 us, 2048 x 8192 770 -> 28 us; one token, 128256 x 2048
 // 1006 -> 172 us (6.1 TB/s); 777 tokens, 2048 x 2048 256 -> 69 us, 2048 x 8192 993 -> 214 us (122 TFLOP/s), SwiGLU 8192 x 2048 1483 ->
 // 356 us (146 TFLOP/s; 331 us before boxes were handed back after the vote and the small products had one shape).
 //
@@ -80,6 +80,7 @@ struct Args {
     int w_stages, x_stages, a_slots;
     int tmem_cols;
     int ring_bytes, x_bytes;             // shared memory: W ring | x pieces | chunk sums (cluster > 1)
+    int sum_cols;                        // the smaller kernel: tokens whose chunk sums are kept (cluster > 1)
 };
 
 __device__ __forceinline__ void give_up_f32(const Args& a, int code) { atomicCAS(a.status, 0, (code << 16) | (int)(blockIdx.x & 0xffff)); }
@@ -404,8 +405,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     for (int j = 0; j < 8; ++j) {
                         float t = __uint_as_float(v[j]);
                         if (seg_end) t += __uint_as_float(w[j]);
-                        if (a.cluster > 1) sums[((size_t)c * a.tt + col0 + g + j) * kRows + row] = t;
-                        else total[g + j] += t;
+                        if (a.cluster > 1) {
+                            if (!SMALL || col0 + g + j < a.sum_cols) sums[((size_t)c * (SMALL ? a.sum_cols : a.tt) + col0 + g + j) * kRows + row] = t;
+                        } else {
+                            total[g + j] += t;
+                        }
                     }
                 }
             }
@@ -455,7 +459,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const int rows = a.swiglu ? kRows / 2 : kRows, live = tok_end - tok0;
         const int all_chunks = (a.steps + CHUNK - 1) / CHUNK;
         const int per_block = a.segs / a.cluster * (a.seg_steps / CHUNK);         // (the last block may have fewer)
-        const int l = (threadIdx.x >> 3) & 3, per_pass = blockDim.x / 4, stride = a.tt * kRows;
+        const int l = (threadIdx.x >> 3) & 3, per_pass = blockDim.x / 4, stride = (SMALL ? a.sum_cols : a.tt) * kRows;
         for (int e0 = rank * per_pass; e0 < live * rows; e0 += a.cluster * per_pass) {
             const int e = e0 + (threadIdx.x >> 5) * 8 + (threadIdx.x & 7);
             const int col = min(e / rows, live - 1), row = e % rows;             // (all lanes take part in the sums)
@@ -505,8 +509,12 @@ struct Plan { int tt, cluster, w_stages, x_stages, a_slots, tmem_cols, smem; };
 
 // The cut of a product into tiles of `tt` tokens and clusters over the k range: the one with the least estimated clocks.  A step of
 // 64 k costs a block the larger of its tensor-core time (12 clocks a token) and its shared-memory time (64 KiB of W written and
-// read, 1152 bytes a token, at 128 bytes a clock), and about 1000 clocks of barriers whatever its size; blocks that share an SM share
-// the former two.  Listed form: `listed` tiles are expected, of `tokens` rows at most.
+// read, 1152 bytes a token, at 128 bytes a clock), and about 1000 clocks of barriers whatever its size.
+// Few tokens (at most 16): a step is a chain of barriers of 1280 clocks, of 1500 for each of two blocks on an SM; the weights arrive at 3400
+// bytes a clock of the whole GPU; the sums of a cluster are kept for the tokens there are, which leaves an SM room for two blocks.  Of clusters of
+// eight that fill their SMs by themselves only fourteen run at a time (the SMs of a GPC are no multiple of eight): 5 x 2048 x 8192 took
+// 34 us that way, the last two clusters starting 15 us late, and 28 with two blocks an SM; 5 x 3072 x 2048 in clusters of eight instead of four 14 -> 11.
+// Listed form: `listed` tiles are expected, of `tokens` rows at most.
 Plan make_plan(int tokens, int n, int swiglu, int steps, int seg_steps, int sms, int listed) {
     const int segs = (steps + seg_steps - 1) / seg_steps;
     const bool small = tokens <= kSmallTokens;
@@ -520,7 +528,7 @@ Plan make_plan(int tokens, int n, int swiglu, int steps, int seg_steps, int sms,
             const long long ctas = f_tiles * (listed ? listed : (tokens + tt - 1) / tt) * cl;
             const int cta_steps = segs / cl * seg_steps < steps ? segs / cl * seg_steps : steps;
             const int chunks = (cta_steps + kChunkSteps - 1) / kChunkSteps;
-            const int sums = cl > 1 ? chunks * tt * kRows * 4 : 0, x_stage = 3 * tt * 128;
+            const int sums = cl > 1 ? chunks * (small ? tokens : tt) * kRows * 4 : 0, x_stage = 3 * tt * 128;
             // two blocks an SM where their sums leave the rings room
             bool two = small && 4 * tt + 2 * kACols <= 256;
             auto w_stages = [&](int xs) {
@@ -535,8 +543,14 @@ Plan make_plan(int tokens, int n, int swiglu, int steps, int seg_steps, int sms,
             const double mma = 12.0 * tt, smem_clk = (65536.0 + 1152.0 * tt) / 128.0, barriers = 1000.0;
             const double per_sm = (double)((ctas + sms - 1) / sms);
             const double step_clk = mma > smem_clk ? mma : smem_clk;
-            const double cost = per_sm * (cta_steps * (step_clk > barriers || two ? step_clk : barriers) + 3000.0) +
+            double cost = per_sm * (cta_steps * (step_clk > barriers ? step_clk : barriers) + 3000.0) +
                                 (cl > 1 ? 2000.0 + 40.0 * chunks * cl * tt / 16 : 0.0);
+            if (small) {
+                const long long slots = two ? 2LL * sms : cl == 8 ? 14 * 8 : sms;
+                const double chain = (double)((ctas + slots - 1) / slots) * cta_steps * (two && ctas > sms ? 1500.0 : 1280.0);
+                const double stream = (double)(ctas / cl) * kRows * steps * kStepK * 4.0 / 3400.0;
+                cost = (chain > stream ? chain : stream) + 3000.0 + (cl > 1 ? 2000.0 + 40.0 * chunks * cl : 0.0);
+            }
             if (cost < best_cost) {
                 best_cost = cost;
                 const int cols = two || 4 * tt + 2 * kACols <= 256 ? 256 : 512, slots = (cols - 4 * tt) / kACols;
@@ -592,6 +606,7 @@ int run(const float* x, const int* source, const float* w, int tokens, int group
     a.ring_bytes = p.w_stages * kBoxBytes;
     a.x_bytes = p.x_stages * 3 * p.tt * 128;
     a.tmem_cols = p.tmem_cols;
+    a.sum_cols = tile_tokens;
     a.t_tiles = max_tiles ? max_tiles : (tokens + p.tt - 1) / p.tt;
     const long long blocks_x = (long long)(a.swiglu ? (a.n + 63) / 64 : (a.n + kRows - 1) / kRows) * a.t_tiles * p.cluster;
     if (blocks_x > 0x7fffffffLL) LLM_FAIL(-1, "gemm_f32_tc: %d tokens by %d are too many for one launch", tokens, a.n);
