@@ -26,9 +26,23 @@ __device__ __forceinline__ void load2(const __nv_bfloat16* p, float& a, float& b
     b = v.y;
 }
 
+// Sums over the block as 256 threads take them (block_sum's order), whatever the block's size: `v` of the first 256 threads counts.
+__device__ __forceinline__ float sum_of_256(float v, float* scratch) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    v = warp_sum(v);
+    __syncthreads();  // scratch may still be read from an earlier call
+    if (lane == 0 && warp < 8) scratch[warp] = v;
+    __syncthreads();
+    return warp_sum(lane < 8 ? scratch[lane] : 0.f);
+}
+
 // TAPS > 0: the number of taps is known when compiling (the loops over taps unroll to exactly that many); 0: any number.
-template <typename T, int TAPS>
-__global__ void __launch_bounds__(256)
+// FEW: for few tokens, 1024 threads instead of 256 to a token, since a block's own width is all the parallelism there is; the squares
+// are then summed out of shared memory by 256 threads, in the order of the other form (the same bits).  One token of 6144 channels and
+// four taps: 27 -> 12.7 us; the taps, the state and the products' row are 190 KiB through one SM.
+constexpr int kFewTokens = 148;      // a block of 1024 threads to an SM
+template <typename T, int TAPS, bool FEW>
+__global__ void __launch_bounds__(FEW ? 1024 : 256)
 conv_norm_store_kernel(const T* __restrict__ u, const float* __restrict__ bias, const float* __restrict__ taps_w, int taps_any,
                        const float* __restrict__ q_gain, const float* __restrict__ k_gain,
                        const float* __restrict__ state, const int* __restrict__ state_slots,
@@ -84,8 +98,19 @@ conv_norm_store_kernel(const T* __restrict__ u, const float* __restrict__ bias, 
             }
             y[c] = a0;
             y[c + 1] = a1;
-            if (c < cq) ssq += a0 * a0 + a1 * a1;
-            else if (c < cq + ck) ssk += a0 * a0 + a1 * a1;
+            if (!FEW) {
+                if (c < cq) ssq += a0 * a0 + a1 * a1;
+                else if (c < cq + ck) ssk += a0 * a0 + a1 * a1;
+            }
+        }
+        if (FEW) {
+            __syncthreads();
+            if (threadIdx.x < 256)
+                for (int c = 2 * threadIdx.x; c < cq + ck; c += 512) {
+                    const float a0 = y[c], a1 = y[c + 1];
+                    if (c < cq) ssq += a0 * a0 + a1 * a1;
+                    else ssk += a0 * a0 + a1 * a1;
+                }
         }
     } else {
         for (int c = threadIdx.x; c < channels; c += blockDim.x) {
@@ -102,16 +127,26 @@ conv_norm_store_kernel(const T* __restrict__ u, const float* __restrict__ bias, 
                 acc = to_f32(u[(size_t)t * channels + c]) + bc;
             }
             y[c] = acc;
-            if (c < cq) ssq += acc * acc;
-            else if (c < cq + ck) ssk += acc * acc;
+            if (!FEW) {
+                if (c < cq) ssq += acc * acc;
+                else if (c < cq + ck) ssk += acc * acc;
+            }
+        }
+        if (FEW) {
+            __syncthreads();
+            if (threadIdx.x < 256)
+                for (int c = threadIdx.x; c < cq + ck; c += 256) {
+                    if (c < cq) ssq += y[c] * y[c];
+                    else ssk += y[c] * y[c];
+                }
         }
     }
-    const float tq = block_sum(ssq, red);
+    const float tq = FEW ? sum_of_256(ssq, red) : block_sum(ssq, red);
     const float inv_q = 1.0f / sqrtf(tq / (float)cq + eps);
     for (int c = threadIdx.x; c < cq; c += blockDim.x)
         q_out[(size_t)t * cq + c] = from_f32<T>(y[c] * inv_q * q_gain[c]);
     if (!cache) return;
-    const float tk = block_sum(ssk, red);
+    const float tk = FEW ? sum_of_256(ssk, red) : block_sum(ssk, red);
     const float inv_k = 1.0f / sqrtf(tk / (float)ck + eps);
     const int slot = slots[t];
     const int page = slot / page_size, off = slot % page_size;
@@ -184,9 +219,10 @@ LLM_API int llm_conv_norm_store(const void* u, const float* bias, const float* t
         using T = decltype(tag);
 #define LLM_CONV(TT)                                                                                                       \
     do {                                                                                                                   \
-        if (smem > 48 * 1024)                                                                                              \
-            cudaFuncSetAttribute(conv_norm_store_kernel<T, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
-        llm_launch(conv_norm_store_kernel<T, TT>, tokens, 256, smem, stream, (const T*)u, bias, taps_w, taps, q_gain, k_gain, \
+        const bool few = tokens <= kFewTokens;                                                                             \
+        const auto kern = few ? conv_norm_store_kernel<T, TT, true> : conv_norm_store_kernel<T, TT, false>;                \
+        if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
+        llm_launch(kern, tokens, few ? 1024 : 256, smem, stream, (const T*)u, bias, taps_w, taps, q_gain, k_gain,           \
                    (const float*)state, state_slots, token_request, cu_seqlens, (T*)q_out, (T*)cache, slots, page_stride,   \
                    page_size, heads, kv_heads, dim, vdim, channels, eps);                                                   \
     } while (0)

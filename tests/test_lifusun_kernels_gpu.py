@@ -75,6 +75,31 @@ def test_conv_norm_store(K, dtype, heads, kv_heads, dim, vdim, taps, own):
         assert torch.equal(st[1], state[1])                # a slot of no request of the step is left alone
 
 
+# a token by 1024 threads (few tokens) and by 256 (many): the same bits; channels below and beyond a round of either, odd ones, no keys
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,taps,own", [(32, 8, 128, 128, 4, True), (3, 1, 5, 7, 3, True), (16, 4, 40, 24, 1, True), (9, 3, 128, 64, 2, False)])
+def test_conv_norm_store_of_few_tokens(K, dtype, heads, kv_heads, dim, vdim, taps, own):
+    n, many, page = 5, 200, 16
+    C = heads * dim + (kv_heads * (dim + vdim) if own else 0)
+    g = torch.Generator(device=DEV).manual_seed(C)
+    u = torch.randn(n, C, generator=g, device=DEV).to(dtype).repeat(many // n, 1)         # requests of one token: every fifth is alike
+    bias, taps_w = torch.randn(C, generator=g, device=DEV), torch.randn(C, taps, generator=g, device=DEV)
+    qg, kg = torch.rand(heads * dim, generator=g, device=DEV) + 0.5, torch.rand(kv_heads * dim, generator=g, device=DEV) + 0.5
+    state = torch.randn(n, taps - 1, C, generator=g, device=DEV).repeat(many // n, 1, 1) if taps > 1 else None
+    got = []
+    for rows in (many, n):
+        cache = torch.zeros(-(-rows // page), kv_heads * page * (dim + vdim), device=DEV, dtype=dtype) if own else None
+        q = torch.empty(rows, heads * dim, device=DEV, dtype=dtype)
+        at = i32(list(range(rows)))
+        K.conv_norm_store(u[:rows].contiguous(), bias, taps_w, qg, kg if own else None, state.clone() if taps > 1 else None, at, at, i32(list(range(rows + 1))),
+                          q, cache, at if own else None, heads, kv_heads, dim, vdim, 1e-5)
+        kp = cache[0, :kv_heads * page * dim].view(kv_heads, page, dim)[:, :n] if own else None
+        vp = cache[0, kv_heads * page * dim:].view(kv_heads, page, vdim)[:, :n] if own else None
+        got.append((q[:n], kp, vp))
+    for a, b in zip(*got):
+        assert a is None or torch.equal(a, b)
+
+
 def paged_case(dtype, heads, kv_heads, dim, vdim, page, seqs, seed=0):
     """Keys and values of `seqs` = [(context length, rows of the step)] in shuffled pages; every request brings its last rows."""
     g = torch.Generator().manual_seed(seed)
