@@ -5,7 +5,8 @@
 //                   One block per row, the row held in registers between the two passes, sums in a fixed order.
 //                   With a second gain the new residual row is normed as well, into rows of the engine's type: the norm
 //                   in front of the next sub-layer of a design that has norms on both sides of its sub-layers.
-//                   A branch may arrive as the k-split parts of a product (few rows only): they are added in split order as they are read.
+//                   A branch may arrive as the k-split parts of a product (few rows only): they are added in split order as they are read
+//                   and the sum is rounded to the type the product has, so a row does not depend on who adds its parts.
 // llm_rmsnorm_rows: out[t] = in[t] * rsqrt(mean(in[t]^2) + eps) * weight for rows of the engine's type with strides of their
 //                   own (some columns of a wider product), float32 statistics.
 // llm_glu_clamped:  act = g * sigmoid(slope * g) * (u + 1) with g = min(gate, limit), u = clamp(up, -limit, limit),
@@ -123,6 +124,7 @@ norm_add_few_kernel(float* __restrict__ residual, const TB* __restrict__ branch,
 #pragma unroll
             for (int k = 1; k < kMaxParts; ++k)
                 if (k < splits && tid + j * kFewThreads < width) b[j] += e[j][k];
+            b[j] = to_f32(from_f32<TB>(b[j]));             // as a kernel that adds the parts into rows of this type leaves them
         }
     }
     // sums of squares as kNormThreads threads take them: element tid + kNormThreads * j, from round `from` to the row's end, then from 0
@@ -240,14 +242,14 @@ LLM_API int llm_norm_add_few_rows(int width) { return width <= kFewWidth ? kFewR
 
 // branch [tokens, width] of `branch_dtype`; weight float32 or bfloat16 (`weight_dtype`); cast: null or [tokens, width] of
 // `cast_dtype`.  accumulate == 0 writes the normed row instead of adding it (an embedding's norm).  splits > 0: `branch` is float32 parts
-// [splits][tokens][width], `split_stride` numbers apart (at most llm_norm_add_few_rows() rows, of at most 4096 numbers).
+// [splits][tokens][width], `split_stride` numbers apart, of rows of `branch_dtype` (at most llm_norm_add_few_rows() rows, of at most 4096 numbers).
 LLM_API int llm_norm_add(float* residual, const void* branch, int branch_dtype, const void* weight, int weight_dtype,
                          void* cast, int cast_dtype, int tokens, int width, float eps, int accumulate, const void* next_weight,
                          void* next_out, int splits, long long split_stride, cudaStream_t stream) {
     if (tokens == 0) return 0;
     if (width <= 0) LLM_FAIL(-1, "norm_add: width %d", width);
     const bool few = tokens <= kFewRows && width <= kFewWidth;
-    if (splits < 0 || splits > kMaxParts || (splits > 0 && (!few || branch_dtype != LLM_F32)))
+    if (splits < 0 || splits > kMaxParts || (splits > 0 && !few))
         LLM_FAIL(-1, "norm_add: %d parts of %d rows of %d numbers are not taken", splits, tokens, width);
     if ((next_weight == nullptr) != (next_out == nullptr)) LLM_FAIL(-1, "norm_add: the second norm needs a gain and a place for its rows");
     return llm_dispatch_dtype(branch_dtype, [&](auto tb) {

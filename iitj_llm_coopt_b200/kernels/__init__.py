@@ -1005,10 +1005,11 @@ class Kernels:
         """residual (+)= rmsnorm(branch) * weight with float32 statistics (csrc/branch_norm.cu); `cast_out`: a copy of the new
         residual in another type (what the next sub-layer reads).  `accumulate` False writes the normed rows instead.
         With `next_weight` and `next_out` the new residual rows are normed too: next_out = rmsnorm(residual) * next_weight.
-        `branch` may be a PartialSums: the parts of few rows are added while they are read."""
+        `branch` may be a PartialSums: the parts of few rows are added while they are read, and rounded to the type of its `out`
+        as `materialize` would (the same bits)."""
         _check(residual, "norm_add.residual", torch.float32, 2)
         tokens, width = residual.shape
-        splits, stride = 0, 0
+        splits, stride, branch_dtype = 0, 0, branch.dtype
         if isinstance(branch, PartialSums) and branch.splits <= 8 and tokens <= self.lib.llm_norm_add_few_rows(width):
             _need(tuple(branch.shape) == (tokens, width), "norm_add: shapes differ")
             splits, stride, branch = branch.splits, branch.stride, branch.parts[0]
@@ -1027,7 +1028,7 @@ class Kernels:
                   "norm_add.next_out: shape or type differs")
         else:
             _need(next_weight is None, "norm_add: a second gain without a place for its rows")
-        self._call("llm_norm_add", _ptr(residual), _ptr(branch), DTYPE_CODE[branch.dtype], _ptr(weight), DTYPE_CODE[weight.dtype],
+        self._call("llm_norm_add", _ptr(residual), _ptr(branch), DTYPE_CODE[branch_dtype], _ptr(weight), DTYPE_CODE[weight.dtype],
                    _ptr(cast_out), DTYPE_CODE[typed.dtype] if typed is not None else 0, tokens, width, float(eps),
                    1 if accumulate else 0, _ptr(next_weight), _ptr(next_out), splits, stride, self._stream())
         return residual

@@ -340,8 +340,9 @@ def test_planted_keys_at_the_window_s_edges(K, dtype, window, page, total):
             assert (want[:, :vdim].amax(1) > 1.0).any()       # the planted value shows in the answer
 
 
-# few rows (a block of 1024 threads a row, the parts of a product added as they are read) against many (256 threads a row) and the
-# restatement: one thread's number, the edges of the rounds of 256 and 1024, the widest row that few rows take, one more
+# few rows (a block of 1024 threads a row, the parts of a product added as they are read and rounded to the product's type) against
+# their sum by a kernel of its own, against many rows (256 threads a row) and the restatement: one thread's number, the edges of the
+# rounds of 256 and 1024, the widest row that few rows take, one more
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("tokens,width,splits", [(1, 8, 2), (3, 1024, 8), (148, 1028, 3), (2, 2052, 5), (5, 3072, 1), (1, 4096, 8), (2, 4100, 4), (149, 512, 2)])
 def test_norm_add_of_parts(K, dtype, tokens, width, splits):
@@ -352,19 +353,56 @@ def test_norm_add_of_parts(K, dtype, tokens, width, splits):
     total = parts[0].clone()
     for p in parts[1:]:
         total += p
+    total = total.to(dtype)
+    assert torch.equal(PartialSums(K, parts, torch.empty_like(total)).sum(), total)
+
+    def norm_add(branch, residual, accumulate):
+        out = [residual.clone()] + [torch.empty(residual.shape, device="cuda", dtype=dtype) for _ in range(2)]
+        K.norm_add(out[0], branch, w, 1e-5, cast_out=out[1], accumulate=accumulate, next_weight=w2, next_out=out[2])
+        return out
     for accumulate in (True, False):
-        got, cast, nxt = res.clone(), torch.empty(tokens, width, device="cuda", dtype=dtype), torch.empty(tokens, width, device="cuda", dtype=dtype)
-        K.norm_add(got, PartialSums(K, parts, torch.empty_like(total)), w, 1e-5, cast_out=cast, accumulate=accumulate, next_weight=w2, next_out=nxt)
+        got, cast, nxt = norm_add(PartialSums(K, parts, torch.empty_like(total)), res, accumulate)
         want = R.ref_norm_add(res, total, w, 1e-5, accumulate)
         assert ((got - want).norm() / want.norm()).item() < 1e-6          # (two sums of `width` numbers in float32)
-        assert torch.equal(cast, got.to(dtype))
         unit = got.double() * torch.rsqrt(got.double().pow(2).mean(1, keepdim=True) + 1e-5) * w2
         assert ((nxt - unit).norm() / unit.norm()).item() < (1e-6 if dtype == torch.float32 else 2.0 ** -8)
+        for a, b in zip((got, cast, nxt), norm_add(total, res, accumulate)):
+            assert torch.equal(a, b)
         rows = 160                                                          # the same rows among many: the same bits
-        if tokens < rows and width <= 4096:
-            many, big = res.repeat(rows, 1)[:rows].contiguous(), total.repeat(rows, 1)[:rows].contiguous()
-            K.norm_add(many, big, w, 1e-5, accumulate=accumulate)
-            assert torch.equal(many[:tokens], got)
+        if tokens < rows:
+            many = norm_add(total.repeat(rows, 1)[:rows].contiguous(), res.repeat(rows, 1)[:rows].contiguous(), accumulate)
+            for a, b in zip((got, cast, nxt), many):
+                assert torch.equal(a, b[:tokens])
+
+
+# whole steps in bfloat16: the same logits whether the parts of the output products are added by the norm that reads them or by a kernel of
+# their own (the norms of these families are behind the sub-layers, and a unit head of wkv amplifies a rounding)
+@pytest.mark.parametrize("shape,layers", [("rodapel-1b", 4), ("fomerax-1b", 4)])
+def test_deferred_sums_change_no_logits(K, monkeypatch, shape, layers):
+    from iitj_llm_coopt_b200 import LLM, StepEntry
+    from iitj_llm_coopt_b200.config.registry import architecture_for
+    from iitj_llm_coopt_b200.presets import shape_config
+    cfg = shape_config(shape)
+    cfg["layers"] = cfg["layers"][:layers]
+    typed = architecture_for(cfg).config_class.from_dict(cfg)
+    deferred = []
+    norm_add = K.norm_add
+    monkeypatch.setattr(K, "norm_add", lambda residual, branch, *a, **k: (deferred.append(not isinstance(branch, torch.Tensor)),
+                                                                         norm_add(residual, branch, *a, **k))[1])
+    for seed in (1, 2):
+        got = []
+        for defer in (True, False):
+            monkeypatch.setattr(K, "defer_sums", defer)
+            deferred.clear()
+            llm = LLM(config=typed, random_seed=seed, dtype="bfloat16", page_size=16, max_num_seqs=8, num_pages=8, max_num_batched_tokens=64, max_model_len=64)
+            runner, cache = llm.engine.runner, llm.engine.cache
+            cache.admit("r")
+            tokens = torch.randint(0, 500, (40,), generator=torch.Generator().manual_seed(seed)).tolist()
+            got.append([runner.step([StepEntry("r", tokens[:35], [34])]).clone()] + [runner.step([StepEntry("r", [t], [0])]).clone() for t in tokens[35:]])
+            assert any(deferred) == defer
+            del llm, runner, cache
+        for a, b in zip(*got):
+            assert torch.equal(a, b)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
