@@ -426,7 +426,7 @@ int launch_few(const void* q, int q_stride, const void* cache, long long page_st
     int threads = (own * (vdim / 2) + 31) / 32 * 32;
     if (threads < 128) threads = 128;
     const size_t smem = sizeof(float) * (2 * (size_t)heads * kSpan + (size_t)own * kSpan + ((heads * own + 3) & ~3) + (size_t)own * dim);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(talking_attn_few_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    LLM_ALLOW_SMEM("talking_attention", talking_attn_few_kernel<T>, smem);
     llm_launch_cluster(talking_attn_few_kernel<T>, (unsigned)(tokens * cluster), threads, smem, stream, (unsigned)cluster, (const T*)q, q_stride,
                        (const T*)cache, page_stride, v_off, block_table, table_width, token_request, positions, talk, slopes, (T*)out,
                        out_stride, heads, kv_heads, dim, vdim, page_size, chunk, scale, cluster);
@@ -442,8 +442,7 @@ int launch_talking(const void* q, int q_stride, const void* cache, long long pag
     const int warps = (heads + HPW - 1) / HPW;
     const size_t smem = sizeof(float) * ((((size_t)heads * dim + 3) & ~(size_t)3) + (size_t)heads * ((heads + 7) & ~7) + (size_t)heads * kTile);
     if (smem > 200 * 1024) LLM_FAIL(-1, "talking attention: %d heads of %d dims do not fit shared memory", heads, dim);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(talking_attn_kernel<T, HPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    LLM_ALLOW_SMEM("talking_attention", (talking_attn_kernel<T, HPW>), smem);
     llm_launch(talking_attn_kernel<T, HPW>, tokens, warps * 32, smem, stream, (const T*)q, q_stride, (const T*)cache,
                page_stride, v_off, block_table, table_width, token_request, positions, talk, slopes, (T*)out, out_stride,
                heads, kv_heads, dim, vdim, page_size, chunk, scale, vec);

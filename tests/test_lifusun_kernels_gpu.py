@@ -170,10 +170,11 @@ def test_talking_attention_tiles_on_the_tensor_core(K, heads, kv_heads, dim, vdi
 
 
 # a cluster a token (up to 64 tokens) against a block a token (more) and the restatement: one to eight heads a block, clusters of four and
-# eight, one tile and many rounds of two tiles, positions at, before and behind the edges of tiles, rounds and chunks, values of the lowest width
+# eight, one tile and many rounds of two tiles, positions at, before and behind the edges of tiles, rounds and chunks, values of the lowest width; and 64 heads of 384 numbers,
+# which want 48 KiB of shared memory beside the kernel's own
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim,page,chunk", [(32, 8, 128, 128, 16, 64), (8, 4, 96, 80, 16, 48), (24, 8, 64, 64, 16, 0), (4, 4, 16, 8, 8, 24),
-                                                                (12, 3, 40, 256, 4, 100), (64, 8, 32, 128, 16, 0), (20, 5, 8, 16, 4, 8)])
+                                                                (12, 3, 40, 256, 4, 100), (64, 8, 32, 128, 16, 0), (20, 5, 8, 16, 4, 8), (64, 8, 384, 128, 16, 64)])
 def test_talking_attention_of_few_tokens(K, dtype, heads, kv_heads, dim, vdim, page, chunk):
     lengths = [1, 2, 31, 32, 33, 63, 64, 65, 96, 97, 127, 128, 129, 200, 47, 48, 49, 24, 25, 100, 101]
     seqs = [(n, 1) for n in lengths + [150] * 50]
