@@ -221,7 +221,7 @@ LLM_API int llm_conv_norm_store(const void* u, const float* bias, const float* t
     do {                                                                                                                   \
         const bool few = tokens <= kFewTokens;                                                                             \
         const auto kern = few ? conv_norm_store_kernel<T, TT, true> : conv_norm_store_kernel<T, TT, false>;                \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
+        LLM_ALLOW_SMEM("conv_norm_store", kern, smem);                                                                     \
         llm_launch(kern, tokens, few ? 1024 : 256, smem, stream, (const T*)u, bias, taps_w, taps, q_gain, k_gain,           \
                    (const float*)state, state_slots, token_request, cu_seqlens, (T*)q_out, (T*)cache, slots, page_stride,   \
                    page_size, heads, kv_heads, dim, vdim, channels, eps);                                                   \
