@@ -118,7 +118,7 @@ LLM_API int llm_add_branch_rmsnorm(float* residual, const void* delta, int delta
                 constexpr int F = decltype(form_tag)::value;
                 if (!vec) {
                     auto kern = branch_rmsnorm_kernel<TD, TO, F>;
-                    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                    if (llm_smem_opt_in(smem)) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                     llm_launch(kern, (unsigned)out_rows, 256, smem, stream, residual, d, factor, rows, gain, (TO*)out, width, eps);
                     return;
                 }

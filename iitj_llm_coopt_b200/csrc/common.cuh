@@ -97,9 +97,10 @@ __device__ __forceinline__ float4 sum_parts4(const float* p, int splits, size_t 
 // Lets `kern` have `bytes` of dynamic shared memory.  A kernel's static shared memory counts toward the 48 KiB that need no
 // opt-in: at most 8 KiB are allowed for here (a kernel of 64 heads of 384 numbers asked for exactly 48 KiB beside its own 1 KiB, and
 // its launch was refused).
+static inline bool llm_smem_opt_in(size_t bytes) { return bytes + 8 * 1024 > 48 * 1024; }
 #define LLM_ALLOW_SMEM(name, kern, bytes)                                                                                     \
     do {                                                                                                                      \
-        if ((size_t)(bytes) + 8 * 1024 > 48 * 1024) {                                                                         \
+        if (llm_smem_opt_in(bytes)) {                                                                                         \
             const cudaError_t e_ = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes));     \
             if (e_ != cudaSuccess) LLM_FAIL(-2, "%s: %zu bytes of shared memory: %s", name, (size_t)(bytes), cudaGetErrorString(e_)); \
         }                                                                                                                     \

@@ -266,10 +266,7 @@ LLM_API int llm_add_rmsnorm(float* residual, const void* delta, const int* rows,
                 return 0;
             }
             auto kern = add_rmsnorm_kernel<TD, TW>;
-            if (smem > 48 * 1024) {
-                cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                if (e != cudaSuccess) LLM_FAIL(-2, "add_rmsnorm: %s", cudaGetErrorString(e));
-            }
+            LLM_ALLOW_SMEM("add_rmsnorm", kern, smem);
             llm_launch(kern, out_rows, 256, smem, stream, residual, (const TD*)delta, rows, (const TW*)weight,
                                                   (TD*)out, width, eps, splits, (size_t)split_stride);
             LLM_CHECK_LAUNCH("add_rmsnorm");

@@ -678,7 +678,7 @@ int run_step(StepArgs& a, int dtype, int requests, cudaStream_t stream) {
             int threads = (a.ds * ((per + cols - 1) / cols) + 31) / 32 * 32;
             threads = threads < 128 ? 128 : threads > 512 ? 512 : threads;
             const size_t smem = sizeof(float) * (2 * (size_t)a.ds * 4 * sp.pieces + 2 * (size_t)per);
-            if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (llm_smem_opt_in(smem)) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (a.slices > 1)
                 llm_launch_cluster(kern, dim3((unsigned)(requests * a.slices), (unsigned)a.heads), threads, smem, stream, (unsigned)a.slices, a);
             else
@@ -703,7 +703,7 @@ int run_walk(WalkArgs& a, int dtype, int n_walks, cudaStream_t stream) {
         auto go = [&](auto kern, int cols) {
             const int cpb = 128 / a.ds * cols;
             const size_t smem = sizeof(float) * kStage * (2 * (size_t)a.ds * 4 * sp.pieces + cpb + 3);
-            if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (llm_smem_opt_in(smem)) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             llm_launch(kern, dim3((unsigned)((columns + cpb - 1) / cpb), (unsigned)a.heads, (unsigned)n_walks), 128, smem, stream, a);
         };
         if (sp.pieces == 1) go(state_walk_kernel<T, KIND, 1, 2>, 2);

@@ -136,7 +136,7 @@ LLM_API int llm_post_norm(const float* x, const void* branch, int branch_dtype, 
         using TB = decltype(tb);
         return llm_dispatch_dtype(cast ? cast_dtype : LLM_BF16, [&](auto tc) {
             using TC = decltype(tc);
-            if (smem > 48 * 1024) cudaFuncSetAttribute(post_norm_kernel<TB, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            LLM_ALLOW_SMEM("post_norm", (post_norm_kernel<TB, TC>), smem);
             llm_launch(post_norm_kernel<TB, TC>, (unsigned)tokens, kThreads, smem, stream, x, (const TB*)branch, alpha, gain, eps, out,
                        (TC*)cast, history, mix, inputs, entry_stride, width);
             LLM_CHECK_LAUNCH("post_norm");

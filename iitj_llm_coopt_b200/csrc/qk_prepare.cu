@@ -123,7 +123,7 @@ LLM_API int llm_qk_prepare(void* row, int ld, const float* bias, const float* q_
     if (smem > 200 * 1024) LLM_FAIL(-1, "qk_prepare: a row of %zu bytes does not fit shared memory", smem);
     return llm_dispatch_dtype(dtype, [&](auto tag) {
         using T = decltype(tag);
-        if (smem > 48 * 1024) cudaFuncSetAttribute(qk_prepare_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        LLM_ALLOW_SMEM("qk_prepare", qk_prepare_kernel<T>, smem);
         llm_launch(qk_prepare_kernel<T>, (unsigned)tokens, 256, smem, stream, a);
         LLM_CHECK_LAUNCH("qk_prepare");
         return 0;

@@ -45,7 +45,7 @@ def test_embed(K, dtype, vocab, width, tokens):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("wdtype", DTYPES)
-@pytest.mark.parametrize("rows,width,eps", [(5, 96, 1e-6), (19, 200, 1e-5), (3, 4104, 1e-5), (2, 13000, 1e-5)])
+@pytest.mark.parametrize("rows,width,eps", [(5, 96, 1e-6), (19, 200, 1e-5), (3, 4104, 1e-5), (2, 12287, 1e-5), (2, 13000, 1e-5)])
 def test_add_rmsnorm(K, dtype, wdtype, rows, width, eps):
     res = rnd((rows, width), torch.float32, 2)
     delta = rnd((rows, width), dtype, 3)

@@ -174,7 +174,7 @@ def test_matrix_memory_at_the_gates_ends(K, dtype, f_bias):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("T,width", [(1, 64), (5, 320), (9, 4096), (600, 384), (7, 50), (600, 50)])
+@pytest.mark.parametrize("T,width", [(1, 64), (5, 320), (9, 4096), (600, 384), (7, 50), (600, 50), (2, 12287)])
 @pytest.mark.parametrize("form", ["rows", "float32 rows", "parts", "routed", "routed and rows", "routed and parts"])
 def test_add_branch_rmsnorm(K, dtype, T, width, form):
     from iitj_llm_coopt_b200.kernels import PartialSums

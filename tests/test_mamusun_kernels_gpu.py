@@ -42,6 +42,7 @@ def tables_for(pos, rot, amp=1.0):
     (2, 2, 8, 6, "none", False, True, 4, True, True, True, False, 8),           # a bias on the values too
     (1, 1, 130, 70, "head", False, True, 130, False, False, True, False, 32),   # a whole wide head rotates
     (64, 8, 128, 128, "row", True, True, 64, False, True, True, True, 16),      # a row beyond 48 KB of shared memory
+    (64, 32, 128, 16, "row", True, True, 64, False, True, True, False, 16),      # a row of 48 KB beside the kernel's own shared memory
 ])
 def test_qk_prepare(K, dtype, heads, kv_heads, dim, vdim, norm, gains, norm_first, rot, inter, bias, own, vfk, page):
     lens = [37, 5]
@@ -167,7 +168,7 @@ def test_planted_scores_show_the_sink_and_the_window_s_edge(K, dtype, page, wind
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("tokens,width,inputs", [(1, 8, 2), (5, 200, 3), (3, 2050, 7), (2, 13000, 2)])
+@pytest.mark.parametrize("tokens,width,inputs", [(1, 8, 2), (5, 200, 3), (3, 2050, 7), (2, 12288, 2), (2, 13000, 2)])
 def test_post_norm_and_the_average_over_depth(K, dtype, tokens, width, inputs):
     x, branch, gain = rnd(tokens, width, seed=1), rnd(tokens, width, dtype=dtype, seed=2, s=3.0), rnd(width, seed=3) * 0.1 + 1.0
     for alpha in (1.0, 3.5):
