@@ -225,7 +225,7 @@ attn_f32_single_kernel(const float* __restrict__ q, int q_stride, const float* _
     float* Vs = smem_f;                                // [kStages][32][D]
     __shared__ __align__(16) float qs[D], p[kSpan];
     __shared__ float tile_max[kSpan / 32], tile_sum[kSpan / 32], tile_corr[kSpan / 32];
-    const int t = items ? items[blockIdx.y] : (int)blockIdx.y, h = blockIdx.x, hk = h / (heads / kv_heads);
+    const int t = items[blockIdx.y], h = blockIdx.x, hk = h / (heads / kv_heads);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int pos = positions[t], lo = window > 0 ? max(0, pos - window + 1) : 0;
     const int* table = block_table + (size_t)token_request[t] * table_width;
@@ -357,7 +357,7 @@ LLM_API int llm_attention_f32_tiles(const float* q, int q_stride, const float* c
     return head_dim == 64 ? go(attn_f32_tile_kernel<64>, tile_smem<64>()) : go(attn_f32_tile_kernel<128>, tile_smem<128>());
 }
 
-// items: the token rows of single decoded tokens (null: rows 0 .. n_items - 1).
+// items: the token rows of single decoded tokens.
 LLM_API int llm_attention_f32_single(const float* q, int q_stride, const float* cache, const int* block_table, int table_width,
                                      const int* items, int n_items, const int* token_request, const int* positions, float* out,
                                      int out_stride, int heads, int kv_heads, int head_dim, int page_size, int window, float scale,

@@ -1360,23 +1360,23 @@ class Kernels:
             if splits > 1:
                 self.launches += 1      # the merge kernel
             return out
-        if q.dtype == torch.float32 and plan is not None and tokens <= 65535 and q.shape[1] % 4 == 0 and \
+        lists = () if plan is None else [plan.device_arrays.get(n) for n in ("items", "runs")]
+        if q.dtype == torch.float32 and any(x is not None for x in lists) and tokens <= 65535 and q.shape[1] % 4 == 0 and \
                 self.flat_f32_runs(heads, kv_heads, key_dim, value_dim, shared_value) and \
                 gate is None and slopes is None and sinks is None and every == 0 and softcap == 0 and \
                 not (q.data_ptr() | out.data_ptr() | cache_layer.data_ptr()) & 15:
-            # plain scores over planes of one size: the kernels of float32 attention, whose sums are the general kernel's, in its order (a
-            # token behind 337 keys, 32 heads on 8 of 64 numbers, took 200 us there: one warp walks all keys of a head)
-            if getattr(plan, "single", False):
-                self._call("llm_attention_f32_single", _ptr(q), q.shape[1], _ptr(cache_layer), _ptr(meta.block_table),
-                           meta.block_table.shape[1], None, tokens, _ptr(meta.token_request), _ptr(meta.positions), _ptr(out),
-                           out.shape[1], heads, kv_heads, key_dim, page_size, int(window), float(scale), self._stream())
-                return out
-            runs = plan.device_arrays.get("runs")
+            # plain scores over planes of one size: the kernels of float32 attention, whose sums are the general kernel's, in its order,
+            # where the step's plan found them the faster ones
+            items, runs = lists
             if runs is not None:
                 self._call("llm_attention_f32_tiles", _ptr(q), q.shape[1], _ptr(cache_layer), _ptr(meta.block_table),
                            meta.block_table.shape[1], _ptr(runs), runs.shape[0] // 4, _ptr(out), out.shape[1], heads, kv_heads, key_dim,
                            page_size, int(window), float(scale), self._stream())
-                return out
+            if items is not None:
+                self._call("llm_attention_f32_single", _ptr(q), q.shape[1], _ptr(cache_layer), _ptr(meta.block_table),
+                           meta.block_table.shape[1], _ptr(items), items.shape[0], _ptr(meta.token_request), _ptr(meta.positions), _ptr(out),
+                           out.shape[1], heads, kv_heads, key_dim, page_size, int(window), float(scale), self._stream())
+            return out
         self._call("llm_attention_flat", _ptr(q), q.shape[1], _ptr(cache_layer), cache_layer.shape[1], _ptr(meta.block_table),
                    meta.block_table.shape[1], _ptr(meta.token_request), _ptr(meta.positions), _ptr(gate), gate_cols, _ptr(out),
                    out.shape[1], DTYPE_CODE[q.dtype], tokens, heads, kv_heads, key_dim, value_dim, 1 if shared_value else 0, page_size,

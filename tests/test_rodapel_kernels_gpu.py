@@ -416,16 +416,21 @@ def test_glu_clamped_pieces(K, dtype, tokens, inner):
     assert ((out - want).norm() / want.norm()).item() < (1e-6 if dtype == torch.float32 else 2.0 ** -8)
 
 
-# float32, keys and values of one size: with a plan the kernels of float32 attention serve it (csrc/attention_f32.cu), without one the general
-# kernel: the same bits.  Portions that start and end inside tiles of 32 keys and runs of 64 queries, single tokens, windows; and sizes
-# and options that stay with the general kernel
-@pytest.mark.parametrize("heads,kv_heads,dim,vdim,window,page,option", [(8, 2, 64, 64, 0, 16, ""), (4, 4, 128, 128, 50, 8, ""), (6, 2, 64, 64, 33, 4, ""),
+# float32, keys and values of one size: with a plan the kernels of float32 attention serve it (csrc/attention_f32.cu) where they are the faster
+# ones, without one the general kernel: the same bits.  Portions that start and end inside tiles of 32 keys and runs of 64 queries beside single
+# tokens, single tokens alone, windows; many tokens behind few keys, and sizes and options that stay with the general kernel
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,window,page,option", [(8, 2, 64, 64, 0, 16, ""), (4, 4, 128, 128, 50, 8, ""), (6, 2, 64, 64, 33, 4, ""), (6, 2, 64, 64, 100, 4, ""),
                                                                       (4, 2, 64, 128, 0, 16, ""), (4, 2, 32, 32, 0, 16, ""), (4, 2, 64, 64, 0, 16, "gate"),
                                                                       (4, 2, 64, 64, 0, 16, "softcap"), (4, 2, 64, 64, 0, 16, "sinks")])
-def test_flat_attention_in_float32_by_plan(K, heads, kv_heads, dim, vdim, window, page, option):
+def test_flat_attention_in_float32_by_plan(K, monkeypatch, heads, kv_heads, dim, vdim, window, page, option):
     from iitj_llm_coopt_b200.parts.base import StepShape
     from iitj_llm_coopt_b200.parts.flat_tiles import plan_flat_tiles
-    for portions in ([(130, 130), (40, 7), (1, 1), (200, 65)], [(1, 1), (32, 1), (33, 1), (64, 1), (199, 1), (200, 1)]):
+    calls, call = [], K._call
+    monkeypatch.setattr(K, "_call", lambda name, *args: (calls.append(name), call(name, *args))[1])
+    for portions, names in (([(130, 130), (40, 7), (1, 1), (200, 65)], ["items", "runs"]), ([(200, 3), (40, 9)], ["runs"]),
+                            ([(1, 1), (32, 1), (33, 1), (64, 1), (199, 1), (200, 1)], ["items"]), ([(8, 1)] * 600, [])):
+        if not (dim == vdim and dim >= 64) or 0 < window < 64 and len(names) == 2:     # (runs of 64 walk more keys than a row's window has)
+            names = []
         ends, lens = [e for e, _ in portions], [n for _, n in portions]
         cache, table = paged(torch.float32, len(ends), ends, page, kv_heads * (dim + vdim), seed=dim)
         cache.copy_(rnd(*cache.shape, seed=3))
@@ -435,10 +440,14 @@ def test_flat_attention_in_float32_by_plan(K, heads, kv_heads, dim, vdim, window
         q = rnd(T, heads * dim, seed=5)
         more = {"gate": {"gate": rnd(T, heads, seed=6)}, "softcap": {"softcap": 5.0}, "sinks": {"sinks": rnd(heads, seed=7)}}.get(option, {})
         plan = plan_flat_tiles(K, StepShape(lens, ends, T, False, False, "cuda"), heads, kv_heads, dim, vdim, window, dtype=torch.float32)
+        assert sorted(plan.arrays) == names + ["tiles"] and plan.graph_key == (plan.splits, bool(names))
         plan.bind({n: torch.tensor(v, dtype=torch.int32).cuda() for n, v in plan.arrays.items()})
         out, want = torch.full((T, heads * vdim), 7.0, device="cuda"), torch.empty(T, heads * vdim, device="cuda")
         K.attention_flat(q, cache, meta, want, heads, kv_heads, dim, vdim, window=window, scale=0.2, **more)
+        calls.clear()
         K.attention_flat(q, cache, meta, out, heads, kv_heads, dim, vdim, window=window, scale=0.2, plan=plan, **more)
+        kernels = [{"items": "llm_attention_f32_single", "runs": "llm_attention_f32_tiles"}[n] for n in reversed(names) if not option]
+        assert calls == (kernels or ["llm_attention_flat"])
         assert torch.equal(out, want)
         exact = torch.empty(T, heads * vdim, dtype=torch.float32, device="cuda")
         R.TorchKernels().attention_flat(q, cache, meta, exact, heads, kv_heads, dim, vdim, window=window, scale=0.2, **more)
