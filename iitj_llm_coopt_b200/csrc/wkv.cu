@@ -88,8 +88,12 @@ wkv_decay_kernel(const float* __restrict__ low, const float* __restrict__ w2, co
 }
 
 // Few tokens: a channel a thread, its row of W2 asked for while the kernel ahead finishes, 64 channels a block.  The sum over j in order, as above.
-// (The kernel above stages W2 piece by piece behind barriers: one token of 3072 channels and rank 64 took 13 us.)
+// (The kernel above stages W2 piece by piece behind barriers: one token of 3072 channels and rank 64 takes 7.2 us there, 2.4 here, eight 8.0 and 4.0.)
+// Every token reads W2 again, so it pays for a few blocks to an SM, fewer where a row of W2 is longer than what is asked for ahead twice over:
+// rank 64, 768 blocks (24 x 2048) 9.1 -> 8.7 us, 864 (18 x 3072) 9.2 -> 7.4, but 1024 (32 x 2048) 9.2 -> 9.8 and 1152 (24 x 3072) 9.2 -> 10.1; rank 128
+// and 1024, 576 blocks 15.2 -> 11.1 (9 x 4096) and 111 -> 80 (12 x 3072), but 768 15.6 -> 17.1 (12 x 4096) and 117 -> 129 (16 x 3072).
 constexpr int kFewTokens = 32, kFewChannels = 64, kFewAhead = 8;       // kFewAhead: loads of 16 bytes in flight
+constexpr int few_blocks_of(int rank) { return (rank <= 2 * 4 * kFewAhead ? 6 : 4) * 148; }
 
 __global__ void __launch_bounds__(kFewChannels)
 wkv_decay_few_kernel(const float* __restrict__ low, const float* __restrict__ w2, const float* __restrict__ w0, float* __restrict__ out,
@@ -248,9 +252,9 @@ LLM_API int llm_wkv_decay(const float* low, const float* w2, const float* w0, fl
                           cudaStream_t stream) {
     if (tokens == 0) return 0;
     // (rows of W2 that start on 16 bytes; a rank whose row fits shared memory without asking)
-    const int few_blocks = (channels + kFewChannels - 1) / kFewChannels;
-    if (tokens <= kFewTokens && rank % 4 == 0 && rank <= 8192 && !((uintptr_t)w2 & 15) && few_blocks <= 65535) {
-        llm_launch(wkv_decay_few_kernel, dim3((unsigned)tokens, few_blocks), kFewChannels, sizeof(float) * rank, stream, low, w2, w0, out, channels, rank);
+    const long long few_blocks = (channels + kFewChannels - 1) / kFewChannels;
+    if (tokens <= kFewTokens && tokens * few_blocks <= few_blocks_of(rank) && rank % 4 == 0 && rank <= 8192 && !((uintptr_t)w2 & 15) && channels > 0) {
+        llm_launch(wkv_decay_few_kernel, dim3((unsigned)tokens, (unsigned)few_blocks), kFewChannels, sizeof(float) * rank, stream, low, w2, w0, out, channels, rank);
         LLM_CHECK_LAUNCH("wkv_decay");
         return 0;
     }

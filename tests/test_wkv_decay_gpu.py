@@ -33,3 +33,18 @@ def test_a_rank_that_one_block_could_not_hold():
     K.wkv_decay(low, w2, w0, out)
     want = torch.exp(-torch.exp(torch.tanh(low.double()) @ w2.double().t() + w0.double()))
     assert (out - want).abs().max().item() < 5e-5
+
+
+# tokens that the kernel of few takes, on both sides of the limits of its rule, against the same rows among many: the same bits
+@pytest.mark.parametrize("tokens,channels,rank", [(1, 1, 4), (5, 63, 8), (5, 65, 64), (18, 3072, 64), (19, 3072, 64), (9, 4096, 128), (10, 4096, 128), (32, 512, 32),
+                                                  (33, 512, 32), (2, 64, 8192), (3, 130, 100), (3, 130, 50)])
+def test_few_tokens_give_the_bits_of_many(tokens, channels, rank):
+    from iitj_llm_coopt_b200 import kernels
+    K = kernels.load()
+    g = torch.Generator(device="cuda").manual_seed(channels + rank)
+    low, w2 = torch.randn((tokens, rank), generator=g, device="cuda"), torch.randn((channels, rank), generator=g, device="cuda") * 0.2
+    w0 = torch.randn(channels, generator=g, device="cuda") - 1.0
+    few, many = torch.full((tokens + 1, channels), 7.0, device="cuda"), torch.empty(tokens + 40, channels, device="cuda")
+    K.wkv_decay(low, w2, w0, few[:tokens])
+    K.wkv_decay(torch.cat([low, torch.zeros(40, rank, device="cuda")]), w2, w0, many)
+    assert torch.equal(few[:tokens], many[:tokens]) and (few[tokens] == 7.0).all()
