@@ -40,7 +40,10 @@ __device__ __forceinline__ float sum_of_256(float v, float* scratch) {
 // FEW: for few tokens, 1024 threads instead of 256 to a token, since a block's own width is all the parallelism there is; the squares
 // are then summed out of shared memory by 256 threads, in the order of the other form (the same bits).  One token of 6144 channels and
 // four taps: 27 -> 12.7 us; the taps, the state and the products' row are 190 KiB through one SM.
-constexpr int kFewTokens = 148;      // a block of 1024 threads to an SM
+// Up to which token count the wide block is the faster one, in us a call of the other form and of this one: 6144 channels 16.1 and 12.3 at one
+// token, 21.9 and 15.9 at 148 (a block to an SM: beyond it both forms come in waves); 1536 channels 7.3 and 7.0 at one, 10.7 and 9.2 at 100,
+// 8.2 and 8.8 at 148; 768 to 1024 channels level up to 64, 8.3 and 8.9 at 100; 512 channels 5.3 and 6.0 at one.
+int few_tokens(int channels) { return channels < 768 ? 0 : channels < 1536 ? 64 : channels < 3072 ? 100 : 148; }
 template <typename T, int TAPS, bool FEW>
 __global__ void __launch_bounds__(FEW ? 1024 : 256)
 conv_norm_store_kernel(const T* __restrict__ u, const float* __restrict__ bias, const float* __restrict__ taps_w, int taps_any,
@@ -219,7 +222,7 @@ LLM_API int llm_conv_norm_store(const void* u, const float* bias, const float* t
         using T = decltype(tag);
 #define LLM_CONV(TT)                                                                                                       \
     do {                                                                                                                   \
-        const bool few = tokens <= kFewTokens;                                                                             \
+        const bool few = tokens <= few_tokens(channels);                                                                   \
         const auto kern = few ? conv_norm_store_kernel<T, TT, true> : conv_norm_store_kernel<T, TT, false>;                \
         LLM_ALLOW_SMEM("conv_norm_store", kern, smem);                                                                     \
         llm_launch(kern, tokens, few ? 1024 : 256, smem, stream, (const T*)u, bias, taps_w, taps, q_gain, k_gain,           \

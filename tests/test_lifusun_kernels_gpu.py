@@ -79,7 +79,7 @@ def test_conv_norm_store(K, dtype, heads, kv_heads, dim, vdim, taps, own):
 # 12288 channels want 48 KiB of shared memory beside the kernel's own
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim,taps,own", [(32, 8, 128, 128, 4, True), (3, 1, 5, 7, 3, True), (16, 4, 40, 24, 1, True), (9, 3, 128, 64, 2, False),
-                                                               (64, 16, 128, 128, 4, True)])
+                                                               (8, 2, 64, 64, 3, True), (64, 16, 128, 128, 4, True)])
 def test_conv_norm_store_of_few_tokens(K, dtype, heads, kv_heads, dim, vdim, taps, own):
     n, many, page = 5, 200, 16
     C = heads * dim + (kv_heads * (dim + vdim) if own else 0)
