@@ -84,7 +84,12 @@ norm_add_kernel(float* __restrict__ residual, const TB* __restrict__ branch, con
 // 8.3 us there.  With the other kernels of few rows (token shift 21 us, head norms 11.7, wkv decays 13) and the product's parts read here instead of
 // added by a kernel ahead, a prompt of 1111 tokens and eight decode steps at the Rodapel 3B sizes went from 7.41 to 6.77 ms.
 constexpr int kFewThreads = 1024, kFewPer = 4, kFewWidth = kFewThreads * kFewPer;
-constexpr int kFewRows = 148;        // a block is a row and half an SM: beyond a wave of SMs the small blocks are as fast
+constexpr int kFewRows = 148;        // a block of 1024 threads to an SM
+
+// From which width on the wide block is the faster one, in us a call of the other kernel and of this one: bfloat16 branch without a second norm 2.3 and
+// 2.1 (768 numbers, 8 rows), 5.5 and 2.6 (3072, 148 rows), but 1.8 and 2.0 (512, one row); float32 2.4 and 2.3 (1536), 3.6 and 2.5 (3072, 148 rows), but
+// 1.8 and 2.2 (512); with a second norm 4.4 and 3.5 (3072, 148 rows), 3.0 and 3.0 (1536), but 2.4 and 2.8 (512, 37 rows).
+int few_width(int branch_dtype, bool second) { return second ? 2048 : branch_dtype == LLM_BF16 ? 768 : 1536; }
 
 template <typename TB, typename TW, typename TC>
 __global__ void __launch_bounds__(kFewThreads)
@@ -258,7 +263,7 @@ LLM_API int llm_norm_add(float* residual, const void* branch, int branch_dtype, 
             using TW = decltype(tw);
             return llm_dispatch_dtype(cast || next_out ? cast_dtype : LLM_BF16, [&](auto tc) {
                 using TC = decltype(tc);
-                if (few)
+                if (splits > 0 || (few && width >= few_width(branch_dtype, next_out != nullptr)))
                     llm_launch(norm_add_few_kernel<TB, TW, TC>, (unsigned)tokens, kFewThreads, sizeof(float) * width, stream, residual,
                                (const TB*)branch, (const TW*)weight, (TC*)cast, width, eps, accumulate, (const TW*)next_weight, (TC*)next_out,
                                splits, (size_t)split_stride);
