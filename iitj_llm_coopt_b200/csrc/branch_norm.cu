@@ -202,40 +202,50 @@ __global__ void glu_act_kernel(const T* __restrict__ gu, T* __restrict__ act, in
     }
 }
 
-// Eight neighbouring numbers a thread where `vec` (rows and their halves start on 16 bytes), else one.  (A division of 64 bits for every
-// number and one number a load: 1111 rows of 8192 took 33 us.)
+__device__ __forceinline__ float glu_clamped(float g, float u, float limit, float slope) {
+    g = fminf(g, limit);
+    u = fminf(fmaxf(u, -limit), limit);
+    return g / (1.0f + expf(-slope * g)) * (u + 1.0f);
+}
+
 template <typename T>
-__global__ void __launch_bounds__(256)
-glu_clamped_kernel(const T* __restrict__ gu, T* __restrict__ act, int tokens, int inner, float limit, float slope, int vec) {
+__global__ void glu_clamped_kernel(const T* __restrict__ gu, T* __restrict__ act, int tokens, int inner, float limit, float slope) {
     pdl_trigger();
     pdl_wait();
-    auto f = [&](float g, float u) {
-        g = fminf(g, limit);
-        u = fminf(fmaxf(u, -limit), limit);
-        return g / (1.0f + expf(-slope * g)) * (u + 1.0f);
-    };
+    const size_t n = (size_t)tokens * inner;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t t = i / inner, c = i % inner;
+        act[i] = from_f32<T>(glu_clamped(to_f32(gu[t * 2 * inner + c]), to_f32(gu[t * 2 * inner + inner + c]), limit, slope));
+    }
+}
+
+// Eight neighbouring numbers a thread, for rows and halves of rows that start on 16 bytes, and a row of blocks a token (the kernel above divides in
+// 64 bits for every number and loads one at a time).  us in bfloat16, above and here: 1111 rows of 8192 26.4 and 11.7, 37 of 8192 2.2 and 1.8, 148
+// of 2048 2.2 and 2.0, but 16 of 8192 1.7 and 1.8, 8 of 2048 1.3 and 1.8.
+constexpr size_t kGluVec = 200000;         // numbers from which on there are threads enough for all SMs
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+glu_clamped_vec_kernel(const T* __restrict__ gu, T* __restrict__ act, int tokens, int inner, float limit, float slope) {
+    pdl_trigger();
+    pdl_wait();
+    constexpr int kPieces = sizeof(T) / 2;           // 16-byte loads of eight numbers
     for (int t = blockIdx.y; t < tokens; t += gridDim.y) {
         const T* gr = gu + (size_t)t * 2 * inner;
         T* ar = act + (size_t)t * inner;
-        const int first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
-        if (vec) {
-            constexpr int kPieces = sizeof(T) / 2;           // 16-byte loads of eight numbers
-            for (int c = first; c < inner / 8; c += step) {
-                uint4 g[kPieces], u[kPieces], a[kPieces];
+        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < inner / 8; c += gridDim.x * blockDim.x) {
+            uint4 g[kPieces], u[kPieces], a[kPieces];
 #pragma unroll
-                for (int e = 0; e < kPieces; ++e) {
-                    g[e] = reinterpret_cast<const uint4*>(gr + 8 * c)[e];
-                    u[e] = reinterpret_cast<const uint4*>(gr + inner + 8 * c)[e];
-                }
-                const T *gp = reinterpret_cast<const T*>(g), *up = reinterpret_cast<const T*>(u);
-                T* ap = reinterpret_cast<T*>(a);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) ap[e] = from_f32<T>(f(to_f32(gp[e]), to_f32(up[e])));
-#pragma unroll
-                for (int e = 0; e < kPieces; ++e) reinterpret_cast<uint4*>(ar + 8 * c)[e] = a[e];
+            for (int e = 0; e < kPieces; ++e) {
+                g[e] = reinterpret_cast<const uint4*>(gr + 8 * c)[e];
+                u[e] = reinterpret_cast<const uint4*>(gr + inner + 8 * c)[e];
             }
-        } else {
-            for (int c = first; c < inner; c += step) ar[c] = from_f32<T>(f(to_f32(gr[c]), to_f32(gr[inner + c])));
+            const T *gp = reinterpret_cast<const T*>(g), *up = reinterpret_cast<const T*>(u);
+            T* ap = reinterpret_cast<T*>(a);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) ap[e] = from_f32<T>(glu_clamped(to_f32(gp[e]), to_f32(up[e]), limit, slope));
+#pragma unroll
+            for (int e = 0; e < kPieces; ++e) reinterpret_cast<uint4*>(ar + 8 * c)[e] = a[e];
         }
     }
 }
@@ -307,12 +317,14 @@ LLM_API int llm_glu_act(const void* gu, void* act, int dtype, int tokens, int in
 LLM_API int llm_glu_clamped(const void* gu, void* act, int dtype, int tokens, int inner, float limit, float slope,
                             cudaStream_t stream) {
     if (tokens == 0 || inner == 0) return 0;
-    const int vec = inner % 8 == 0 && !(((uintptr_t)gu | (uintptr_t)act) & 15);
-    const int work = vec ? inner / 8 : inner, threads = work < 256 ? (work + 31) / 32 * 32 : 256;
-    const dim3 grid((work + threads - 1) / threads, tokens < 65535 ? tokens : 65535);
+    const size_t n = (size_t)tokens * inner;
+    const bool vec = inner % 8 == 0 && !(((uintptr_t)gu | (uintptr_t)act) & 15) && n >= kGluVec;
+    const int work = inner / 8, threads = vec && work < 256 ? (work + 31) / 32 * 32 : 256;
+    const dim3 grid = vec ? dim3((work + threads - 1) / threads, tokens < 65535 ? tokens : 65535)
+                          : dim3((unsigned)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16));
     return llm_dispatch_dtype(dtype, [&](auto tag) {
         using T = decltype(tag);
-        llm_launch(glu_clamped_kernel<T>, grid, threads, 0, stream, (const T*)gu, (T*)act, tokens, inner, limit, slope, vec);
+        llm_launch(vec ? glu_clamped_vec_kernel<T> : glu_clamped_kernel<T>, grid, threads, 0, stream, (const T*)gu, (T*)act, tokens, inner, limit, slope);
         LLM_CHECK_LAUNCH("glu_clamped");
         return 0;
     });

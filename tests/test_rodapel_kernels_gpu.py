@@ -406,7 +406,7 @@ def test_deferred_sums_change_no_logits(K, monkeypatch, shape, layers):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("tokens,inner", [(1, 8), (3, 100), (2, 2056), (70, 8192)])
+@pytest.mark.parametrize("tokens,inner", [(1, 8), (3, 100), (2, 2056), (70, 8192), (70, 8191), (3000, 100), (49, 4104), (48, 4104), (70000, 8)])
 def test_glu_clamped_pieces(K, dtype, tokens, inner):
     gu = (2.0 * torch.randn(tokens, 2 * inner, generator=torch.Generator(device="cuda").manual_seed(inner), device="cuda")).to(dtype)
     out = torch.empty(tokens, inner, device="cuda", dtype=dtype)
