@@ -507,13 +507,26 @@ constexpr int kSmemLimit = 226 * 1024;      // of 227 KiB a block; the static ar
 
 struct Plan { int tt, cluster, w_stages, x_stages, a_slots, tmem_cols, smem; };
 
+// Clusters of 1 to 8 blocks that run at a time: one block to an SM as cudaOccupancyMaxActiveClusters gives it (the SMs of a GPC are no multiple of
+// eight), two to an SM as the times below fit it.
+constexpr int kClusters[2][9] = {{0, 148, 74, 45, 33, 26, 22, 15, 15}, {0, 296, 148, 90, 74, 52, 44, 30, 35}};
+
+// us of a product of at most 16 tokens: `tiles` tiles of 128 features in clusters of `cl` blocks of `cta_steps` steps each, `per_sm` blocks to an SM.
+// A wave is a chain of barriers (1.1 us a step where two blocks share an SM) and, in a cluster, a pass over the sums for every `cl` tokens; the waves
+// and the stream of the weights hide in each other for the most part.  Fitted to 939 cuts of 30 products (n 512 to 50000, k 512 to 18944) at 1, 4, 8, 12
+// and 16 tokens; the cut it takes is 0.3 % off the fastest on average, 9 % at most.  (An estimate without the passes and with one block to an SM only
+// where two don't fit was 7.6 % off, 16 x 14000 x 1500 2.2 times: 48.7 us for 21.7.  16 x 12000 x 5000 77 -> 57 us, one token by 9000 x 3000 32 -> 26,
+// by 2048 x 8192 24, by 18944 x 3584 65 -> 45.)
+double few_us(long long tiles, int cl, int cta_steps, int per_sm, int tokens, int steps) {
+    const long long waves = (tiles + kClusters[per_sm - 1][cl] - 1) / kClusters[per_sm - 1][cl];
+    const double sums = cl > 1 ? 1.2 + 1.9 * ((tokens + cl - 1) / cl - 1) : 0.0;
+    const double chain = waves * (cta_steps * (per_sm == 2 ? 1.08 : 0.59) + 6.6 + sums), stream = tiles * kRows * steps * kStepK * 4.0 / 5.8e6 + 1.5;
+    return chain > stream ? chain + 0.34 * stream : stream + 0.34 * chain;
+}
+
 // The cut of a product into tiles of `tt` tokens and clusters over the k range: the one with the least estimated clocks.  A step of
 // 64 k costs a block the larger of its tensor-core time (12 clocks a token) and its shared-memory time (64 KiB of W written and
-// read, 1152 bytes a token, at 128 bytes a clock), and about 1000 clocks of barriers whatever its size.
-// Few tokens (at most 16): a step is a chain of barriers of 1280 clocks, of 1500 for each of two blocks on an SM; the weights arrive at 3400
-// bytes a clock of the whole GPU; the sums of a cluster are kept for the tokens there are, which leaves an SM room for two blocks.  Of clusters of
-// eight that fill their SMs by themselves only fourteen run at a time (the SMs of a GPC are no multiple of eight): 5 x 2048 x 8192 took
-// 34 us that way, the last two clusters starting 15 us late, and 28 with two blocks an SM; 5 x 3072 x 2048 in clusters of eight instead of four 14 -> 11.
+// read, 1152 bytes a token, at 128 bytes a clock), and about 1000 clocks of barriers whatever its size.  Few tokens (at most 16): few_us.
 // Listed form: `listed` tiles are expected, of `tokens` rows at most.
 Plan make_plan(int tokens, int n, int swiglu, int steps, int seg_steps, int sms, int listed) {
     const int segs = (steps + seg_steps - 1) / seg_steps;
@@ -523,40 +536,32 @@ Plan make_plan(int tokens, int n, int swiglu, int steps, int seg_steps, int sms,
     double best_cost = 1e30;
     const int most = tokens >= kMaxTile ? kMaxTile : (tokens + 15) / 16 * 16;
     for (int tt = small || listed ? most : 16; tt <= most; tt += 16)
-        for (int cl = 1; cl <= segs; ++cl) {
-            if (segs % cl) continue;
-            const long long ctas = f_tiles * (listed ? listed : (tokens + tt - 1) / tt) * cl;
-            const int cta_steps = segs / cl * seg_steps < steps ? segs / cl * seg_steps : steps;
-            const int chunks = (cta_steps + kChunkSteps - 1) / kChunkSteps;
-            const int sums = cl > 1 ? chunks * (small ? tokens : tt) * kRows * 4 : 0, x_stage = 3 * tt * 128;
-            // two blocks an SM where their sums leave the rings room
-            bool two = small && 4 * tt + 2 * kACols <= 256;
-            auto w_stages = [&](int xs) {
-                const int room = ((two ? 112 * 1024 : kSmemLimit) - 1024 - sums - xs * x_stage) / kBoxBytes / 2 * 2;
-                return room < kMaxW ? room : kMaxW;
-            };
-            if (two && w_stages(2) < 4) two = false;
-            const int ws = w_stages(2);
-            if (ws < 4) continue;
-            int xs = 2;
-            while (xs < kMaxX && w_stages(xs + 1) == ws) ++xs;
-            const double mma = 12.0 * tt, smem_clk = (65536.0 + 1152.0 * tt) / 128.0, barriers = 1000.0;
-            const double per_sm = (double)((ctas + sms - 1) / sms);
-            const double step_clk = mma > smem_clk ? mma : smem_clk;
-            double cost = per_sm * (cta_steps * (step_clk > barriers ? step_clk : barriers) + 3000.0) +
-                                (cl > 1 ? 2000.0 + 40.0 * chunks * cl * tt / 16 : 0.0);
-            if (small) {
-                const long long slots = two ? 2LL * sms : cl == 8 ? 14 * 8 : sms;
-                const double chain = (double)((ctas + slots - 1) / slots) * cta_steps * (two && ctas > sms ? 1500.0 : 1280.0);
-                const double stream = (double)(ctas / cl) * kRows * steps * kStepK * 4.0 / 3400.0;
-                cost = (chain > stream ? chain : stream) + 3000.0 + (cl > 1 ? 2000.0 + 40.0 * chunks * cl : 0.0);
+        for (int cl = 1; cl <= segs; ++cl)
+            for (int per_sm = 1; per_sm <= (small ? 2 : 1); ++per_sm) {
+                if (segs % cl) continue;
+                const long long ctas = f_tiles * (listed ? listed : (tokens + tt - 1) / tt) * cl;
+                const int cta_steps = segs / cl * seg_steps < steps ? segs / cl * seg_steps : steps;
+                const int chunks = (cta_steps + kChunkSteps - 1) / kChunkSteps;
+                const int sums = cl > 1 ? chunks * (small ? tokens : tt) * kRows * 4 : 0, x_stage = 3 * tt * 128;
+                auto w_stages = [&](int xs) {
+                    const int room = ((per_sm == 2 ? 112 * 1024 : kSmemLimit) - 1024 - sums - xs * x_stage) / kBoxBytes / 2 * 2;
+                    return room < kMaxW ? room : kMaxW;
+                };
+                const int ws = w_stages(2);
+                if (ws < 4) continue;
+                int xs = 2;
+                while (xs < kMaxX && w_stages(xs + 1) == ws) ++xs;
+                const double mma = 12.0 * tt, smem_clk = (65536.0 + 1152.0 * tt) / 128.0, barriers = 1000.0;
+                const double step_clk = mma > smem_clk ? mma : smem_clk;
+                const double cost = small ? few_us(ctas / cl, cl, cta_steps, per_sm, tokens, steps)
+                                          : (double)((ctas + sms - 1) / sms) * (cta_steps * (step_clk > barriers ? step_clk : barriers) + 3000.0) +
+                                                (cl > 1 ? 2000.0 + 40.0 * chunks * cl * tt / 16 : 0.0);
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    const int cols = per_sm == 2 || 4 * tt + 2 * kACols <= 256 ? 256 : 512, slots = (cols - 4 * tt) / kACols;
+                    best = Plan{tt, cl, ws, xs, slots < kMaxA ? slots : kMaxA, cols, ws * kBoxBytes + xs * x_stage + sums + 1024};
+                }
             }
-            if (cost < best_cost) {
-                best_cost = cost;
-                const int cols = two || 4 * tt + 2 * kACols <= 256 ? 256 : 512, slots = (cols - 4 * tt) / kACols;
-                best = Plan{tt, cl, ws, xs, slots < kMaxA ? slots : kMaxA, cols, ws * kBoxBytes + xs * x_stage + sums + 1024};
-            }
-        }
     return best;
 }
 

@@ -57,6 +57,19 @@ def test_many_blocks(K, tokens, n, k):
     assert ((out - want).norm() / want.norm()).item() < 1e-6 and K.gemm_status() == 0
 
 
+# few tokens: one block and two to an SM, clusters of one to eight blocks, one wave and several; a row has the same bits in every cut
+@pytest.mark.parametrize("n,k", [(14000, 1500), (9000, 3000), (18944, 3584), (5120, 3072), (2560, 2560), (1536, 1536), (8192, 2048), (768, 768), (20000, 2048)])
+def test_cuts_of_few_tokens(K, n, k):
+    x, w = rnd((16, k), 1), rnd((n, k), 2, k ** -0.5)
+    want, first = product(x, w), None
+    for tokens in (16, 12, 8, 4, 1):
+        out = torch.full((tokens + 1, n), 7.0, device="cuda")
+        K.linear(x[:tokens].contiguous(), w, out[:tokens])
+        assert ((out[:tokens] - want[:tokens]).norm() / want[:tokens].norm()).item() < 1e-6 and K.gemm_status() == 0
+        first = out[:16] if first is None else first
+        assert torch.equal(out[:tokens], first[:tokens]) and (out[tokens] == 7.0).all()
+
+
 def test_infinities_and_nans_go_where_they_would(K):
     x, w = rnd((40, 300), 3), rnd((70, 300), 4)
     x[3, 5], x[4, 299], x[5, 0] = float("inf"), float("nan"), -float("inf")
