@@ -33,7 +33,8 @@ def rnd(shape, dtype, seed, std=1.0):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("vocab,width,tokens", [(320, 96, 7), (1000, 200, 33)])
+# few tokens with a row over several blocks (up to 64) and many, rows of one piece and of twelve, none at all
+@pytest.mark.parametrize("vocab,width,tokens", [(320, 96, 7), (1000, 200, 33), (320, 256, 64), (320, 257, 5), (1000, 3072, 5), (1000, 3072, 65), (320, 0, 3)])
 def test_embed(K, dtype, vocab, width, tokens):
     table = rnd((vocab, width), dtype, 1)
     ids = torch.randint(0, vocab, (tokens,), device="cuda", dtype=torch.int32)
