@@ -262,6 +262,49 @@ def test_latent_prepare_and_attention(K, dtype, heads, dim, rot, rotary, rank, p
             close(out, want, dtype)
 
 
+# few tokens (a warp a head, up to 32 of them, in blocks of their own size) against the same rows among many: the same bits; heads below
+# four warps, between, and more than a block has warps
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,gains", [(40, 8, 64, 32, True), (1, 1, 20, 7, True), (9, 3, 128, 128, False), (32, 32, 40, 8, True)])
+def test_headnorm_store_of_few_tokens(K, dtype, heads, kv_heads, dim, vdim, gains):
+    few, many, page = 5, 160, 16
+    q_gain, k_gain = (rnd(dim, seed=7) + 1.0, rnd(dim, seed=8) + 1.0) if gains else (None, None)
+    qkv = rnd(few, heads * dim + kv_heads * (dim + vdim), dtype=dtype, seed=1)
+    got = []
+    for rows in (few, many):
+        a = qkv.repeat(rows // few, 1)
+        cache = torch.zeros(-(-rows // page), kv_heads * page * (dim + vdim), dtype=dtype, device="cuda")
+        K.headnorm_store(a, q_gain, k_gain, 1e-5, cache, torch.arange(rows, dtype=torch.int32, device="cuda"), heads, kv_heads, dim, vdim)
+        keys, values = cache[0].split([kv_heads * page * dim, kv_heads * page * vdim])
+        got.append((a[:few], keys.view(kv_heads, page, dim)[:, :few], values.view(kv_heads, page, vdim)[:, :few]))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    heads_in = qkv[:, :heads * dim].double().view(few, heads, dim)
+    unit = heads_in * torch.rsqrt(heads_in.pow(2).mean(-1, keepdim=True) + 1e-5) * q_gain.double() if gains else heads_in
+    close(got[0][0][:, :heads * dim], unit.reshape(few, -1), dtype)
+    assert torch.equal(got[0][2].transpose(0, 1).reshape(few, -1), qkv[:, (heads + kv_heads) * dim:])
+
+
+# a row's channels over several blocks (up to 32 tokens) against the same tokens among many: the same bits
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width", [1, 255, 256, 257, 3072])
+def test_token_shift_of_few_tokens(K, dtype, width):
+    x, mu, before = rnd(7, width, dtype=dtype, seed=1), torch.rand(5 * width).cuda(), rnd(4, width, seed=2)
+    got = []
+    for extra in (0, 40):
+        lens = [4, 3] + [extra] * (extra > 0)
+        cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32).cuda()
+        req = torch.tensor([b for b, m in enumerate(lens) for _ in range(m)], dtype=torch.int32).cuda()
+        slots = torch.tensor([2, 0, 1][:len(lens)], dtype=torch.int32).cuda()
+        rows = torch.cat([x, torch.zeros(extra, width, dtype=dtype, device="cuda")])
+        out = torch.empty(5 * rows.shape[0], width, dtype=dtype, device="cuda")
+        K.token_shift(rows, mu, before, slots, req, cu, out)
+        got.append(out.view(5, -1, width)[:, :7])
+    assert torch.equal(got[0], got[1])
+    prev = torch.cat([before[2:3], x[:3].float(), before[0:1], x[4:6].float()])
+    close(got[0], x.float() + (prev - x.float()) * mu.view(5, 1, width), dtype)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads,dim,width,rank", [(4, 40, 160, 12), (1, 7, 20, 3), (3, 64, 96, 40), (2, 100, 64, 8), (4, 32, 50, 5)])
 def test_wkv(K, dtype, heads, dim, width, rank):
