@@ -263,7 +263,9 @@ LLM_API int llm_headnorm_store(void* qkv, int ld, const float* q_gain, const flo
     if (tokens == 0) return 0;
     return llm_dispatch_dtype(dtype, [&](auto tag) {
         using T = decltype(tag);
-        // few tokens: a warp a head instead of four warps that take the heads in turn
+        // Few tokens: a warp a head instead of four warps that take the heads in turn, up to a block of 32 warps to an SM (32 heads of 128, bfloat16:
+        // 1 token 9.1 -> 3.3 us, 148 tokens 9.9 -> 3.5).  Bounds of 128 threads for the many instead of 1024 were slower at most counts (1111 tokens 16.9
+        // and 18.7, float32 4096 43.1 and 52.2; 2048 23.9 and 22.2).
         const int warps = tokens <= 148 ? (heads + kv_heads < 32 ? heads + kv_heads : 32) : 4;
         llm_launch(headnorm_store_kernel<T>, (unsigned)tokens, warps < 4 ? 128 : warps * 32, 0, stream, (T*)qkv, ld, q_gain, k_gain, eps, (T*)cache, slots,
                    page_stride, page_size, heads, kv_heads, dim, vdim);

@@ -239,8 +239,11 @@ __global__ void talking_attn_kernel(const T* __restrict__ q, int q_stride, const
 // round, one pair of output numbers a thread; sums run in the order of the kernel above, tile by tile, and give its bits.
 // 32 heads on 8, chunks of 64, about 27 keys seen, us a call against the kernel above: bfloat16, heads of 128: 1 token 11.3 (in a model with
 // 64 keys 41 before), 32 tokens 16.2, 64 tokens 30.2 against 46.9; heads of 64: 10.9, 16.4, 17.1 against 32.0; float32, heads of 128: 64 tokens 34.1
-// against 68.9.  What is left is the chain: two cluster barriers, the rows of a page table, keys, values.
-constexpr int kFewTokens = 64;                 // 512 blocks: beyond it the clusters come in waves, while a block a token still fits one
+// against 68.9.  What is left is the chain: two cluster barriers, the rows of a page table, keys, values.  Longer ranges keep the distance: without a
+// chunk, 8000 keys, bfloat16, 32 heads of 128: 1 token 5702 -> 1148, 37 tokens 8228 -> 3118; 64 heads of 128, 1000 keys, 64 tokens 1775 -> 1194.
+// Up to 64 tokens it was the faster one at every size timed (8 to 64 heads of 64 and 128, 40 to 8000 keys), by the least for 64 heads of 128 at 64 tokens
+// and 41 keys, where the clusters come in waves: 67.8 -> 61.7.  More tokens have not been timed here.
+constexpr int kFewTokens = 64;
 constexpr int kSpan = 2 * kTile;
 constexpr int kBatch = 16;                     // value rows a thread asks for before it uses the first
 

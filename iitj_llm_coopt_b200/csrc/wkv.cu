@@ -239,7 +239,7 @@ LLM_API int llm_token_shift(const void* x, const float* mu, const float* before,
     if (tokens == 0) return 0;
     return llm_dispatch_dtype(dtype, [&](auto tag) {
         using T = decltype(tag);
-        // few tokens: a channel a thread, a row's channels over several blocks
+        // few tokens: a channel a thread, a row's channels over several blocks (3072 channels, bfloat16: 1 token 8.8 -> 1.9 us, 32 tokens 9.1 -> 3.0)
         const int pieces = tokens <= kFewTokens && width > 256 ? (width + 255) / 256 : 1;
         llm_launch(token_shift_kernel<T>, dim3((unsigned)tokens, pieces < 65535 ? pieces : 65535), 256, 0, stream, (const T*)x, mu, before, state_slots, token_request,
                    cu_seqlens, (T*)out, tokens, width, streams);
